@@ -36,7 +36,7 @@ SOURCES = [
     ("serve.o", "serve.cu", []),
     ("partition.o", "partition.cu", []),
 ]
-HEADERS = ["eb_internal.h", "rod_math.cuh", "bulk_copy.cuh", "contact.h", "eb_host.h", "joint.h"]
+HEADERS = ["eb_internal.h", "rod_math.cuh", "rod_fast.cuh", "bulk_copy.cuh", "contact.h", "eb_host.h", "joint.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -13,27 +13,24 @@
 // table instead).  Every phase loops its threads over the CTA's slots; all
 // per-slot data lives in shared-memory rows, so any thread count works.
 //
-// Step structure: the same substeps as the streaming kernel, including both
-// half drifts of every step, in two phases with one barrier after each (see
-// the step loop).  (Merging the second half drift of step k with
-// the first of step k+1 into one full drift is not an identity here: the
-// reference normalises the rotation axis by theta + 1e-14, so one update by
-// dt differs from two by dt/2 by ~1e-14 per step, which the stiff rod modes
-// amplify into angular-velocity differences far above rounding.  The kernel
-// keeps a compile-time switch for it, unused by the configurations below.)
+// Step structure: the substeps of the streaming kernel in two phases with one
+// barrier after each (element and Voronoi terms; loads, kick and drifts).
 //
 // Rod pairs (kPair): a rod of up to 1039 elements runs on a cluster of two
-// CTAs, each holding half of its slots.  Reads of a neighbouring slot past
-// the left half's end or before the right half's start go to the partner's
-// shared memory (distributed shared memory), and the barriers that order a
-// phase's writes before the next phase's neighbour reads become cluster
-// barriers.  Serving launches mix pairs and single CTAs in one cluster
+// CTAs, each holding half of its slots.  The threads of the slots at the split
+// write what the partner's neighbours read to copies in the partner's shared
+// memory as well (distributed shared memory), so every read is local, and the
+// barriers that order a phase's writes before the next phase's neighbour
+// reads become cluster barriers.  (Reads that go to the partner past the
+// split cost every slot a test and an address, and registers spilled.)  Serving launches mix pairs and single CTAs in one cluster
 // launch; a single CTA takes only CTA barriers.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "eb_internal.h"
-#include "rod_math.cuh"
+#include "rod_fast.cuh"
 
 namespace eb {
 namespace {
@@ -43,62 +40,36 @@ using D3 = Vec3<double>;
 // shared-memory rows (each kCap doubles)
 enum BlockRow : int {
   bX = 0, bV = 3, bQ = 6, bW = 15,  // state (kStateFields rows)
+  // parameters (of the divisors l0 and D0 also the reciprocals, formed once a
+  // launch; explicit damping's rates stay in global memory)
   bMass = 18, bL0 = 19, bD0 = 20, bSig0 = 21, bKap0 = 24, bShear = 27, bBend = 30, bJ = 33, bJinv = 36,
-  bE = 39, bF = 40, bG = 43, bH = 46, bTl = 49,  // per-step exchange rows
-  bNuF = 52, bNuT = 53              // explicit damping only: the last rows, not allocated otherwise
+  bInvL0 = 39, bInvD0 = 40,
+  // exchanged once per force evaluation: internal force of the element, the
+  // couple terms of the Voronoi point
+  bF = 41, bG = 44, bH = 47,
+  // element-local torque terms and dilatation, where a thread steps several slots
+  bTl = 50, bE = 53,
+  kBlockRows = 54
 };
 
-template <int kCap>
+template <int kRow>
 struct BRows {
   double* base;
-  __device__ __forceinline__ double& at(int r, int s) const { return base[r * kCap + s]; }
+  __device__ __forceinline__ double& at(int r, int s) const { return base[r * kRow + s]; }
   __device__ __forceinline__ D3 get3(int r, int s) const {
-    return {base[r * kCap + s], base[(r + 1) * kCap + s], base[(r + 2) * kCap + s]};
+    return {base[r * kRow + s], base[(r + 1) * kRow + s], base[(r + 2) * kRow + s]};
   }
   __device__ __forceinline__ void put3(int r, int s, D3 v) const {
-    base[r * kCap + s] = v.x;
-    base[(r + 1) * kCap + s] = v.y;
-    base[(r + 2) * kCap + s] = v.z;
+    base[r * kRow + s] = v.x;
+    base[(r + 1) * kRow + s] = v.y;
+    base[(r + 2) * kRow + s] = v.z;
   }
 };
 
-// Neighbour access for rod pairs: slot indices at or past `count` continue in
-// the partner's first slots (left half), indices below zero in the partner's
-// last `pcount` slots (right half).
-template <int kCap>
-struct BPair {
-  BRows<kCap> own, peer;
-  int count, pcount;
-  __device__ __forceinline__ double at(int r, int s) const {
-    if (s >= count) return peer.at(r, s - count);
-    if (s < 0) return peer.at(r, s + pcount);
-    return own.at(r, s);
-  }
-  __device__ __forceinline__ D3 get3(int r, int s) const {
-    if (s >= count) return peer.get3(r, s - count);
-    if (s < 0) return peer.get3(r, s + pcount);
-    return own.get3(r, s);
-  }
-};
-
-// parameter field -> shared row (the rows the resident kernel keeps)
-__device__ __forceinline__ int param_row(int f) {
-  switch (f) {
-    case kMass: return bMass;
-    case kL0: return bL0;
-    case kD0: return bD0;
-    case kNuF: return bNuF;
-    case kNuT: return bNuT;
-    default: break;
-  }
-  if (f >= kSig0 && f < kSig0 + 3) return bSig0 + (f - kSig0);
-  if (f >= kKap0 && f < kKap0 + 3) return bKap0 + (f - kKap0);
-  if (f >= kShear && f < kShear + 3) return bShear + (f - kShear);
-  if (f >= kBend && f < kBend + 3) return bBend + (f - kBend);
-  if (f >= kJ && f < kJ + 3) return bJ + (f - kJ);
-  if (f >= kJinv && f < kJinv + 3) return bJinv + (f - kJinv);
-  return -1;  // volume: only read for diagnostics, straight from global memory
-}
+// entries of a row: a CTA of a pair also holds copies of the partner's
+// neighbouring slots, one before its first slot and two after its last
+template <int kCap, bool kPair>
+constexpr int block_row() { return kPair ? kCap + 4 : kCap; }
 
 // kServe: the CTA's slot range, step count, time step and environment come
 // from serve[blockIdx.x] (serving launches)
@@ -109,22 +80,33 @@ __device__ __forceinline__ int param_row(int f) {
 // single CTAs otherwise; without kServe every cluster is a pair
 // kStepper: 0 PositionVerlet, 1 PEFRL (four force evaluations a step), 2
 // VelocityVerlet (two: kick dt/2, drift dt, kick dt/2)
-// FP64 shared-memory rows per slot
-template <bool kDamped>
-constexpr int block_rows() { return kDamped ? 54 : 52; }
-
-// two CTAs per SM for the CTAs of at most 264 slots (420 B a slot undamped)
+// two CTAs per SM for the CTAs of at most 264 slots (437 B a slot)
 template <int kCap>
 constexpr int block_min_ctas() { return kCap <= 264 ? 2 : 1; }
 
-template <int kCap, int kThreads, bool kDamped, bool kSplit, bool kServe, bool kGather = false, bool kPair = false,
+__device__ __forceinline__ double squared_length(D3 d) {
+  return __fma_rn(d.z, d.z, __fma_rn(d.y, d.y, __dmul_rn(d.x, d.x)));
+}
+
+// a slot's state and what its force evaluation hands to its kick
+struct SlotState {
+  D3 x, v, w;
+  double q[9];
+};
+struct SlotTerms {
+  D3 f, g, h, tl;  // internal force of the element, couple terms of the Voronoi point, element-local torque terms
+  double e;        // dilatation
+};
+
+template <int kCap, int kThreads, bool kDamped, bool kServe, bool kGather = false, bool kPair = false,
           int kStepper = 0>
 __global__ void __launch_bounds__(kThreads, block_min_ctas<kCap>()) rod_block_fp64_kernel(const StepArgs a, const int64_t* cta_start,
                                                                     int n_steps_launch, const ServeCta* serve,
                                                                     const int32_t* gmap) {
   extern __shared__ __align__(128) double smem[];
-  const BRows<kCap> R{smem};
-  uint32_t* meta_s = reinterpret_cast<uint32_t*>(smem + block_rows<kDamped>() * kCap);
+  constexpr int kRow = block_row<kCap, kPair>();
+  const BRows<kRow> R{smem + (kPair ? 1 : 0)};
+  uint32_t* meta_s = reinterpret_cast<uint32_t*>(smem + kBlockRows * kRow);
   // per slot: which clamp holds it, the torque, the damper (SlotHits)
   uint8_t* hit_s = reinterpret_cast<uint8_t*>(meta_s + kCap);
 
@@ -151,23 +133,26 @@ __global__ void __launch_bounds__(kThreads, block_min_ctas<kCap>()) rod_block_fp
   }
   if (n_steps <= 0) return;
   const int64_t S = a.stride;
-  // partner rows (its own rows for a single CTA) and cluster barriers
-  BPair<kCap> N{R, R, count, count};
-  bool paired = false;
+  // the partner's rows, at the place of this CTA's slot 0 (left half: past the
+  // end of the right half's left copy; right half: the left half's count)
+  BRows<kRow> peer = R;
+  bool paired = false, left = false;
   if constexpr (kPair) {
     const unsigned partner = blockIdx.x ^ 1u;
+    int pcount = 0;
     if constexpr (kServe) {
       const ServeCta& sc = serve[blockIdx.x];
       const ServeCta& o = serve[partner];
       paired = sc.pair != 0 && o.pair != 0 && sc.steps == o.steps;
-      if (paired) N.pcount = o.count;
+      pcount = o.count;
     } else {
       paired = true;
-      N.pcount = static_cast<int>(cta_start[partner + 1] - cta_start[partner]);
+      pcount = static_cast<int>(cta_start[partner + 1] - cta_start[partner]);
     }
     if (paired) {
       cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-      N.peer.base = cl.map_shared_rank(smem, cl.block_rank() ^ 1u);
+      left = cl.block_rank() == 0;
+      peer.base = cl.map_shared_rank(R.base, cl.block_rank() ^ 1u) + (left ? -count : pcount);
     }
   }
   // orders this phase's writes before the next phase's neighbour reads
@@ -180,72 +165,42 @@ __global__ void __launch_bounds__(kThreads, block_min_ctas<kCap>()) rod_block_fp
     }
     __syncthreads();
   };
-  auto nb3 = [&](int r, int s) -> D3 {
-    if constexpr (kPair) return N.get3(r, s);
-    return R.get3(r, s);
-  };
-  auto nb = [&](int r, int s) -> double {
-    if constexpr (kPair) return N.at(r, s);
-    return R.at(r, s);
-  };
-
   const bool any_rod = (flags & (kSimClamp | kSimDamper | kSimEndTorque)) != 0;
+
+  // global slot of the CTA's slot s
+  auto slot_of = [&](int s) -> int64_t { return kGather ? static_cast<int64_t>(gmap[g0 + s]) : g0 + s; };
 
   // ---- stage state, parameters and slot metadata (coalesced loads)
   for (int s = tid; s < count; s += kThreads) {
-    const int64_t g = kGather ? static_cast<int64_t>(gmap[g0 + s]) : g0 + s;
+    const int64_t g = slot_of(s);
     const uint32_t m = a.meta[g];
     meta_s[s] = m;
     hit_s[s] = static_cast<uint8_t>(any_rod ? slot_hits(a.rods[m >> kRodShift], g) : 0u);
+    // loads in flight together, a group at a time: one CTA fills an SM, so
+    // nothing else hides their latency
+    auto stage = [&](const double* field, int n, int row, auto group) {
+      constexpr int kGroup = decltype(group)::value;
 #pragma unroll 1
-    for (int f = 0; f < kStateFields; ++f) R.at(f, s) = a.in[f * S + g];
-#pragma unroll 1
-    for (int f = 0; f < kParamFields; ++f) {
-      const int r = param_row(f);
-      if (r < 0 || (!kDamped && (f == kNuF || f == kNuT))) continue;
-      R.at(r, s) = a.par[f * S + g];
-    }
-  }
-  __syncthreads();
-
-  // drift of slot s by c (x += c v, Q <- exp(-c [w]x) Q; c = 0 leaves the
-  // slot as it is), then, with `clamp`, the value constraint of the clamp
-  // that holds the slot, if any
-  auto drift = [&](int s, uint32_t meta, double c, bool clamp) {
-    const D3 v = R.get3(bV, s);
-    D3 x = R.get3(bX, s);
-    x = {x.x + c * v.x, x.y + c * v.y, x.z + c * v.z};
-    double q[9];
-    if (meta & kElem) {
+      for (int f = 0; f < n; f += kGroup) {
+        double v[kGroup];
 #pragma unroll
-      for (int k = 0; k < 9; ++k) q[k] = R.at(bQ + k, s);
-      const D3 w = R.get3(bW, s);
-      so3_update_fast(q, c * w.x, c * w.y, c * w.z);
-    }
-    const uint32_t hit = hit_s[s];
-    if (clamp && (hit & (kHitClamp0 | kHitClamp1))) {
-      // the clamp's value constraint: the node, and its element if it has one
-      const RodInfo& ri = a.rods[meta >> kRodShift];
-      const double* tx = (hit & kHitClamp0) ? ri.clamp_x : ri.clamp2_x;
-      const double* tq = (hit & kHitClamp0) ? ri.clamp_Q : ri.clamp2_Q;
-      x = {tx[0], tx[1], tx[2]};
-      if (meta & kElem) {
+        for (int k = 0; k < kGroup; ++k) v[k] = field[(f + k) * S + g];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) q[k] = tq[k];
+        for (int k = 0; k < kGroup; ++k) R.at(row + f + k, s) = v[k];
       }
-    }
-    R.put3(bX, s, x);
-    if (meta & kElem) {
-#pragma unroll
-      for (int k = 0; k < 9; ++k) R.at(bQ + k, s) = q[k];
-    }
-  };
-  // length of element s, rounded as written (so the copy a Voronoi point
-  // recomputes for its next element equals the element's own)
-  auto elem_length = [&](int s) -> double {
-    const D3 dx = nb3(bX, s + 1) - nb3(bX, s);
-    return sqrt(__fma_rn(dx.z, dx.z, __fma_rn(dx.y, dx.y, __dmul_rn(dx.x, dx.x))));
-  };
+    };
+    stage(a.in, kStateFields, bX, std::integral_constant<int, 18>{});
+    // (kSig0 .. kBend and kJ, kJinv are consecutive fields and rows)
+    stage(a.par + kSig0 * S, 12, bSig0, std::integral_constant<int, 12>{});
+    stage(a.par + kJ * S, 6, bJ, std::integral_constant<int, 6>{});
+    const double l0 = a.par[kL0 * S + g], d0 = a.par[kD0 * S + g], m0 = a.par[kMass * S + g];
+    R.at(bL0, s) = l0;
+    R.at(bD0, s) = d0;
+    R.at(bMass, s) = m0;
+    R.at(bInvL0, s) = 1.0 / l0;
+    R.at(bInvD0, s) = 1.0 / d0;
+  }
+  sync_neighbours();
 
   // Substeps: PositionVerlet (drift dt/2, kick dt, drift dt/2), or PEFRL's
   // four kicks with their drifts (in units of dt; compile-time constants)
@@ -258,193 +213,296 @@ __global__ void __launch_bounds__(kThreads, block_min_ctas<kCap>()) rod_block_fp
     return (j == 0 || j == 3) ? 0.5 * (1.0 - 2.0 * kPefrlLambda) : kPefrlLambda;
   };
 
-  // ---- first drift of the first step and the clamp's value constraint
-  // (VelocityVerlet starts with a kick: no drift, the clamp's value alone)
-  for (int s = tid; s < count; s += kThreads)
-    drift(s, meta_s[s], kPefrl ? kPefrlXi * dt : (kVelocity ? 0.0 : hdt), true);
-  sync_neighbours();
+  auto load_state = [&](int s, SlotState& m) {
+    m.x = R.get3(bX, s);
+    m.v = R.get3(bV, s);
+    m.w = R.get3(bW, s);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) m.q[k] = R.at(bQ + k, s);
+  };
+  // the state the neighbours read (their positions, velocities, directors)
+  auto publish = [&](int s, const SlotState& m) {
+    R.put3(bX, s, m.x);
+    R.put3(bV, s, m.v);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) R.at(bQ + k, s) = m.q[k];
+    if (kPair && paired && !left && s < 2) {  // the left half's copies after its last slot
+      peer.put3(bX, s, m.x);
+      peer.put3(bV, s, m.v);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) peer.at(bQ + k, s) = m.q[k];
+    }
+  };
+  // drift of a slot by c (x += c v, Q <- exp(-c [w]x) Q), once or twice:
+  // the closing drift of a step and the first of the next are two rotations
+  // by the same coefficients, formed once and applied one after the other, so a run
+  // rounds alike however it is cut into launches (and one rotation by 2 c
+  // would not be the same: the axis guard of the reference makes it differ by
+  // 1e-14 a step, which stiff rods amplify)
+  auto drift = [&](SlotState& m, uint32_t meta, double c, bool twice) {
+    m.x = {m.x.x + c * m.v.x, m.x.y + c * m.v.y, m.x.z + c * m.v.z};
+    if (twice) m.x = {m.x.x + c * m.v.x, m.x.y + c * m.v.y, m.x.z + c * m.v.z};
+    if (meta & kElem) {
+      const Rotation r = rotation(c * m.w.x, c * m.w.y, c * m.w.z);
+      rotate(m.q, r);
+      if (twice) rotate(m.q, r);
+    }
+  };
+  auto clamp_value = [&](SlotState& m, uint32_t meta, uint32_t hit) {
+    if (!(hit & (kHitClamp0 | kHitClamp1))) return;
+    const RodInfo& ri = a.rods[meta >> kRodShift];
+    const double* tx = (hit & kHitClamp0) ? ri.clamp_x : ri.clamp2_x;
+    const double* tq = (hit & kHitClamp0) ? ri.clamp_Q : ri.clamp2_Q;
+    m.x = {tx[0], tx[1], tx[2]};
+    if (meta & kElem) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) m.q[k] = tq[k];
+    }
+  };
 
-  // Two phases per force evaluation, one barrier after each: (1) element s
-  // (geometry, strain, stress, element-local torque terms) and Voronoi point
-  // s (curvature and couple, with the next element's length recomputed
-  // rather than exchanged); (2) loads, torques, kick and rate constraints,
-  // then the drift before the next force evaluation (after the last kick of
-  // a step: its closing drift and the next step's first, kept apart: merging
-  // them into one rotation is not an identity under the 1e-14 axis guard).
-  for (int step = 0; step < n_steps; ++step)
-  for (int sub = 0; sub < nsub; ++sub) {
-    const double kc = kPefrl ? pefrl_kick(sub) : (kVelocity ? 0.5 : 1.0);  // this kick, in units of dt
+  // Element s (strain, internal force, element-local torque terms) and
+  // Voronoi point s (curvature and couple; the length of element s + 1 is
+  // recomputed rather than exchanged).  The quotients are those of the plain
+  // expressions (rod_fast.cuh): one reciprocal square root gives l and 1 / l,
+  // 1 / e starts from l0 / l and 1 / (e l0) from 1 / l, and division by the
+  // rest lengths uses their stored reciprocals.
+  auto evaluate = [&](int s, uint32_t meta, const SlotState& m, SlotTerms& o) {
+    o.f = o.g = o.h = o.tl = D3{0.0, 0.0, 0.0};
+    o.e = 1.0;
+    if (meta & kElem) {
+      const D3 xn = R.get3(bX, s + 1);
+      const D3 dx = xn - m.x;
+      const Length len = length_of(squared_length(dx));
+      const double l = len.l, il = len.il;
+      const D3 t = {dx.x * il, dx.y * il, dx.z * il};
+      const double l0 = R.at(bL0, s);
+      const double e = div_from(l, l0, R.at(bInvL0, s));
+      const D3 qt = matvec(m.q, t);
+      const D3 sigma = {qt.x * e, qt.y * e, qt.z * e - 1.0};
+      const D3 d = sigma - R.get3(bSig0, s);
+      const D3 sh = R.get3(bShear, s);
+      const D3 nl = {sh.x * d.x, sh.y * d.y, sh.z * d.z};
+      const double ie = rcp_from(e, l0 * il);
+      o.f = scale(mattranspvec(m.q, nl), ie);
+      const D3 J = R.get3(bJ, s);
+      const D3 jwe = {J.x * m.w.x * ie, J.y * m.w.y * ie, J.z * m.w.z * ie};
+      const D3 dv = R.get3(bV, s + 1) - m.v;
+      const double el0 = e * l0;
+      const double rate = div_from(dot(t, dv), el0, rcp_from(el0, il));
+      o.tl = scale(cross(qt, nl), l0) + cross(jwe, m.w) + scale(jwe, rate);
+      o.e = e;
+      if (meta & kVor) {
+        double qn[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) qn[k] = R.at(bQ + k, s + 1);
+        const double D0 = R.at(bD0, s);
+        const D3 kappa = curvature(m.q, qn, D0);
+        const double ln = length_of(squared_length(R.get3(bX, s + 2) - xn)).l;
+        const double eps = div_from(0.5 * (l + ln), D0, R.at(bInvD0, s));
+        const double cube = eps * eps * eps;
+        const double ic = rcp_from(cube, rcp_near(cube));
+        const D3 dk = kappa - R.get3(bKap0, s);
+        const D3 B = R.get3(bBend, s);
+        const D3 tau = {B.x * dk.x, B.y * dk.y, B.z * dk.z};
+        o.g = scale(tau, ic);
+        o.h = scale(cross(kappa, tau), ic * D0);
+      }
+    }
+    R.put3(bF, s, o.f);
+    R.put3(bG, s, o.g);
+    R.put3(bH, s, o.h);
+    if (kPair && paired && left && s == count - 1) {  // the right half's copy before its first slot
+      peer.put3(bF, s, o.f);
+      peer.put3(bG, s, o.g);
+      peer.put3(bH, s, o.h);
+    }
+  };
+
+  // loads, torques, accelerations, kick (by kc dt) and rate constraints
+  // what a slot's kick needs of its mass and its rod's damper
+  struct SlotConst {
+    double im, damper_t, damp;  // 1 / m, exp(-nu_t dt), -nu_r m_e
+  };
+  auto slot_const = [&](int s, int64_t g, uint32_t meta, uint32_t hit) -> SlotConst {
+    const double m = R.at(bMass, s);
+    SlotConst c{1.0 / m, 1.0, 0.0};
+    if (hit & kHitDamper) {
+      const RodInfo& ri = a.rods[meta >> kRodShift];
+      c.damper_t = ri.damper_t;
+      if (meta & kElem) {
+        const double mn = a.par[kMass * S + g + 1];  // the element's other node
+        double em = 0.5 * (m + mn);
+        if (meta & kFirst) em += 0.5 * m;
+        if (meta & kLastElem) em += 0.5 * mn;
+        c.damp = -ri.damper_r * em;
+      }
+    }
+    return c;
+  };
+  // (g: the global slot)
+  auto kick = [&](int s, int64_t g, uint32_t meta, uint32_t hit, const SlotTerms& o, const SlotConst& c, double kc,
+                  SlotState& n) {
+    const bool first = (meta & kFirst) != 0;
     const double kdt = kc == 1.0 ? dt : kc * dt;
     // the damper's time: the kick's share of dt for PEFRL, the full dt for
     // VelocityVerlet (its constants hold dt and act after each kick)
     const double dc = kVelocity ? 1.0 : kc;
     const double ddt = dc == 1.0 ? dt : kdt;
-    for (int s = tid; s < count; s += kThreads) {
-      const uint32_t meta = meta_s[s];
-      D3 f{0.0, 0.0, 0.0}, tl{0.0, 0.0, 0.0};
-      double l = 1.0, e = 1.0;
-      double q[9];
-      if (meta & kElem) {
-#pragma unroll
-        for (int k = 0; k < 9; ++k) q[k] = R.at(bQ + k, s);
-        const D3 dx = nb3(bX, s + 1) - R.get3(bX, s);
-        l = elem_length(s);
-        const double il = 1.0 / l;
-        const D3 t = {dx.x * il, dx.y * il, dx.z * il};
-        const double l0 = R.at(bL0, s);
-        e = l / l0;
-        const D3 qt = matvec(q, t);
-        const D3 sigma = {qt.x * e, qt.y * e, qt.z * e - 1.0};
-        const D3 d = sigma - R.get3(bSig0, s);
-        const D3 sh = R.get3(bShear, s);
-        const D3 nl = {sh.x * d.x, sh.y * d.y, sh.z * d.z};
-        const double ie = 1.0 / e;
-        f = scale(mattranspvec(q, nl), ie);
-        const D3 w = R.get3(bW, s);
-        const D3 J = R.get3(bJ, s);
-        const D3 jwe = {J.x * w.x * ie, J.y * w.y * ie, J.z * w.z * ie};
-        const D3 dv = nb3(bV, s + 1) - R.get3(bV, s);
-        const double rate = dot(t, dv) / (e * l0);
-        tl = scale(cross(qt, nl), l0) + cross(jwe, w) + scale(jwe, rate);
-      }
-      R.at(bE, s) = e;
-      R.put3(bF, s, f);
-      R.put3(bTl, s, tl);
-      D3 gg{0.0, 0.0, 0.0}, hh{0.0, 0.0, 0.0};
-      if (meta & kVor) {
-        double qn[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) qn[k] = nb(bQ + k, s + 1);
-        const double D0 = R.at(bD0, s);
-        const D3 kappa = inv_rotate_divide_fast(q, qn, D0);
-        const double eps = 0.5 * (l + elem_length(s + 1)) / D0;
-        const double ic = 1.0 / (eps * eps * eps);
-        const D3 dk = kappa - R.get3(bKap0, s);
-        const D3 B = R.get3(bBend, s);
-        const D3 tau = {B.x * dk.x, B.y * dk.y, B.z * dk.z};
-        gg = scale(tau, ic);
-        hh = scale(cross(kappa, tau), ic * D0);
-      }
-      R.put3(bG, s, gg);
-      R.put3(bH, s, hh);
+    const double m = R.at(bMass, s);
+    D3 v = n.v, w = n.w;
+    D3 F = o.f;
+    if (!first) F = F - R.get3(bF, s - 1);
+    if (kDamped) {
+      const double cf = m * a.par[kNuF * S + g];
+      F = {F.x - cf * v.x, F.y - cf * v.y, F.z - cf * v.z};
     }
-    sync_neighbours();
-
-    // ---- loads, torques, accelerations, kick, rate constraints
-    for (int s = tid; s < count; s += kThreads) {
-      const uint32_t meta = meta_s[s];
-      const bool first = (meta & kFirst) != 0;
-      const double m = R.at(bMass, s);
-      D3 v = R.get3(bV, s);
-      D3 F = R.get3(bF, s);
-      if (!first) F = F - nb3(bF, s - 1);
-      if (kDamped) {
-        const double cf = m * R.at(bNuF, s);
-        F = {F.x - cf * v.x, F.y - cf * v.y, F.z - cf * v.z};
-      }
-      if (flags & kSimGravity) F = F + D3{gvec[0] * m, gvec[1] * m, gvec[2] * m};
-      const double im = 1.0 / m;
-      v = {v.x + kdt * (F.x * im), v.y + kdt * (F.y * im), v.z + kdt * (F.z * im)};
-      D3 w{0.0, 0.0, 0.0};
-      const uint32_t hit = hit_s[s];
-      const RodInfo* ri = any_rod ? a.rods + (meta >> kRodShift) : nullptr;
-      if (meta & kElem) {
-        const double e = R.at(bE, s);
-        w = R.get3(bW, s);
-        D3 T = R.get3(bG, s);
-        D3 Q2 = R.get3(bH, s);
-        if (!first) {
-          T = T - nb3(bG, s - 1);
-          Q2 = Q2 + nb3(bH, s - 1);
-        }
-        T = T + scale(Q2, 0.5) + R.get3(bTl, s);
-        if (kDamped) {
-          const double ct = 0.5 * (m + nb(bMass, s + 1)) * R.at(bNuT, s);
-          T = {T.x - ct * w.x, T.y - ct * w.y, T.z - ct * w.z};
-        }
-        if (hit & kHitTorque) {
-          double q[9];
-#pragma unroll
-          for (int k = 0; k < 9; ++k) q[k] = R.at(bQ + k, s);
-          T = T + matvec(q, D3{ri->end_torque[0], ri->end_torque[1], ri->end_torque[2]});
-        }
-        const D3 ji = R.get3(bJinv, s);
-        w = {w.x + kdt * (ji.x * T.x * e), w.y + kdt * (ji.y * T.y * e), w.z + kdt * (ji.z * T.z * e)};
-        if (hit & kHitDamper) {
-          const double mn = nb(bMass, s + 1);
-          double em = 0.5 * (m + mn);
-          if (first) em += 0.5 * m;
-          if (meta & kLastElem) em += 0.5 * mn;
-          const double y = -ri->damper_r * em * ddt * e;
-          w = {w.x * exp(y * ji.x), w.y * exp(y * ji.y), w.z * exp(y * ji.z)};
-        }
-      }
-      if (hit & (kHitClamp0 | kHitClamp1)) {
-        v = D3{0.0, 0.0, 0.0};
-        w = D3{0.0, 0.0, 0.0};
-      }
-      // exp(-nu_t dt) for a kick of dt; a fractional kick scales the exponent
-      if (hit & kHitDamper) v = scale(v, dc == 1.0 ? ri->damper_t : exp(log(ri->damper_t) * dc));
-      R.put3(bV, s, v);
-      if (meta & kElem) R.put3(bW, s, w);
-      if (sub + 1 < nsub) {
-        // before the next force evaluation
-        drift(s, meta, kVelocity ? dt : pefrl_pre(sub + 1) * dt, true);
-      } else if (step + 1 < n_steps) {
-        if (kVelocity) {
-          drift(s, meta, 0.0, true);  // the next step starts with a kick: the clamp's value alone
-        } else if (kPefrl) {
-          drift(s, meta, kPefrlXi * dt, false);  // closing drift of this step, own slot
-          drift(s, meta, kPefrlXi * dt, true);   // first drift of the next
-        } else if (kSplit) {
-          drift(s, meta, hdt, false);  // second half of this step, own slot
-          drift(s, meta, hdt, true);   // first half of the next
-        } else {
-          drift(s, meta, dt, true);
-        }
-      }
-    }
-    // the next phase reads the neighbours' drifted state; for a pair, the
-    // partner must also not leave (and free its rows) while this CTA still
-    // reads them
-    sync_neighbours();
-  }
-
-  // ---- closing drift of the last step and write-back
-  const double fin = kPefrl ? kPefrlXi * dt : (kVelocity ? 0.0 : hdt);
-  for (int s = tid; s < count; s += kThreads) {
-    const uint32_t meta = meta_s[s];
-    const int64_t g = kGather ? static_cast<int64_t>(gmap[g0 + s]) : g0 + s;
-    const D3 v = R.get3(bV, s);
-    D3 x = R.get3(bX, s);
-    x = {x.x + fin * v.x, x.y + fin * v.y, x.z + fin * v.z};
-    a.out[kStX * S + g] = x.x;
-    a.out[(kStX + 1) * S + g] = x.y;
-    a.out[(kStX + 2) * S + g] = x.z;
-    a.out[kStV * S + g] = v.x;
-    a.out[(kStV + 1) * S + g] = v.y;
-    a.out[(kStV + 2) * S + g] = v.z;
+    if (flags & kSimGravity) F = F + D3{gvec[0] * m, gvec[1] * m, gvec[2] * m};
+    v = {v.x + kdt * (F.x * c.im), v.y + kdt * (F.y * c.im), v.z + kdt * (F.z * c.im)};
     if (meta & kElem) {
-      double q[9];
-#pragma unroll
-      for (int k = 0; k < 9; ++k) q[k] = R.at(bQ + k, s);
-      const D3 w = R.get3(bW, s);
-      so3_update_fast(q, fin * w.x, fin * w.y, fin * w.z);
-#pragma unroll
-      for (int k = 0; k < 9; ++k) a.out[(kStQ + k) * S + g] = q[k];
-      a.out[kStW * S + g] = w.x;
-      a.out[(kStW + 1) * S + g] = w.y;
-      a.out[(kStW + 2) * S + g] = w.z;
+      const double e = o.e;
+      D3 T = o.g;
+      D3 Q2 = o.h;
+      if (!first) {
+        T = T - R.get3(bG, s - 1);
+        Q2 = Q2 + R.get3(bH, s - 1);
+      }
+      T = T + scale(Q2, 0.5) + o.tl;
+      if (kDamped) {
+        const double ct = 0.5 * (m + a.par[kMass * S + g + 1]) * a.par[kNuT * S + g];
+        T = {T.x - ct * w.x, T.y - ct * w.y, T.z - ct * w.z};
+      }
+      if (hit & kHitTorque) {
+        const RodInfo& ri = a.rods[meta >> kRodShift];
+        T = T + matvec(n.q, D3{ri.end_torque[0], ri.end_torque[1], ri.end_torque[2]});
+      }
+      const D3 ji = R.get3(bJinv, s);
+      w = {w.x + kdt * (ji.x * T.x * e), w.y + kdt * (ji.y * T.y * e), w.z + kdt * (ji.z * T.z * e)};
+      if (hit & kHitDamper) {
+        const double y = c.damp * ddt * e;
+        const double ex = exp(y * ji.x);
+        // (a circular cross section: one factor for both bending directions)
+        w = {w.x * ex, w.y * (ji.y == ji.x ? ex : exp(y * ji.y)), w.z * exp(y * ji.z)};
+      }
     }
+    if (hit & (kHitClamp0 | kHitClamp1)) {
+      v = D3{0.0, 0.0, 0.0};
+      w = D3{0.0, 0.0, 0.0};
+    }
+    // exp(-nu_t dt) for a kick of dt; a fractional kick scales the exponent
+    if (hit & kHitDamper) v = scale(v, dc == 1.0 ? c.damper_t : exp(log(c.damper_t) * dc));
+    n.v = v;
+    n.w = w;
+  };
+  // the drifts between one kick and the next force evaluation, the
+  // constraint's value and the write-out
+  auto advance = [&](int s, uint32_t meta, uint32_t hit, bool last_of_step, int sub, SlotState& m) {
+    if (!last_of_step)
+      drift(m, meta, kVelocity ? dt : pefrl_pre(sub + 1) * dt, false);
+    else if (!kVelocity)  // (VelocityVerlet's next step starts with a kick: the clamp's value alone)
+      drift(m, meta, kPefrl ? kPefrlXi * dt : hdt, true);
+    clamp_value(m, meta, hit);
+    publish(s, m);
+  };
+  // closing drift of the last step and write-back
+  const double fin = kPefrl ? kPefrlXi * dt : (kVelocity ? 0.0 : hdt);
+  auto finish = [&](int64_t g, uint32_t meta, SlotState& m) {
+    if (!kVelocity) drift(m, meta, fin, false);
+    a.out[kStX * S + g] = m.x.x;
+    a.out[(kStX + 1) * S + g] = m.x.y;
+    a.out[(kStX + 2) * S + g] = m.x.z;
+    a.out[kStV * S + g] = m.v.x;
+    a.out[(kStV + 1) * S + g] = m.v.y;
+    a.out[(kStV + 2) * S + g] = m.v.z;
+    if (meta & kElem) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) a.out[(kStQ + k) * S + g] = m.q[k];
+      a.out[kStW * S + g] = m.w.x;
+      a.out[(kStW + 1) * S + g] = m.w.y;
+      a.out[(kStW + 2) * S + g] = m.w.z;
+    }
+  };
+  // Two phases per force evaluation, one barrier after each (for a pair, the
+  // partner must also not leave, and free its rows, while this CTA still
+  // reads them).  A CTA of at most kThreads slots keeps each slot's state and
+  // terms in its thread's registers from phase to phase and launch to end; a
+  // longer one keeps them in their rows.
+  if (count <= kThreads) {
+    const bool on = tid < count;
+    const uint32_t meta = on ? meta_s[tid] : 0u, hit = on ? hit_s[tid] : 0u;
+    int64_t g = 0;
+    SlotConst c;
+    SlotState m;
+    SlotTerms t;
+    if (on) {
+      g = slot_of(tid);
+      c = slot_const(tid, g, meta, hit);
+      load_state(tid, m);
+      // first drift of the first step and the clamp's value constraint
+      // (VelocityVerlet starts with a kick: no drift, the clamp's value alone)
+      if (!kVelocity) drift(m, meta, kPefrl ? kPefrlXi * dt : hdt, false);
+      clamp_value(m, meta, hit);
+      publish(tid, m);
+    }
+    sync_neighbours();
+    for (int step = 0; step < n_steps; ++step)
+      for (int sub = 0; sub < nsub; ++sub) {
+        if (on) evaluate(tid, meta, m, t);
+        sync_neighbours();
+        if (on) {
+          kick(tid, g, meta, hit, t, c, kPefrl ? pefrl_kick(sub) : (kVelocity ? 0.5 : 1.0), m);
+          if (sub + 1 < nsub || step + 1 < n_steps) advance(tid, meta, hit, sub + 1 == nsub, sub, m);
+        }
+        sync_neighbours();
+      }
+    if (on) finish(g, meta, m);
+    return;
+  }
+  for (int s = tid; s < count; s += kThreads) {
+    SlotState m;
+    load_state(s, m);
+    if (!kVelocity) drift(m, meta_s[s], kPefrl ? kPefrlXi * dt : hdt, false);
+    clamp_value(m, meta_s[s], hit_s[s]);
+    publish(s, m);
+  }
+  sync_neighbours();
+  for (int step = 0; step < n_steps; ++step)
+    for (int sub = 0; sub < nsub; ++sub) {
+      for (int s = tid; s < count; s += kThreads) {
+        SlotState m;
+        SlotTerms t;
+        load_state(s, m);
+        evaluate(s, meta_s[s], m, t);
+        R.put3(bTl, s, t.tl);
+        R.at(bE, s) = t.e;
+      }
+      sync_neighbours();
+      for (int s = tid; s < count; s += kThreads) {
+        const uint32_t meta = meta_s[s], hit = hit_s[s];
+        SlotState m;
+        load_state(s, m);
+        const SlotTerms t = {R.get3(bF, s), R.get3(bG, s), R.get3(bH, s), R.get3(bTl, s), R.at(bE, s)};
+        const int64_t g = slot_of(s);
+        kick(s, g, meta, hit, t, slot_const(s, g, meta, hit), kPefrl ? pefrl_kick(sub) : (kVelocity ? 0.5 : 1.0), m);
+        if (sub + 1 < nsub || step + 1 < n_steps)
+          advance(s, meta, hit, sub + 1 == nsub, sub, m);
+        else
+          publish(s, m);
+        R.put3(bW, s, m.w);
+      }
+      sync_neighbours();
+    }
+  for (int s = tid; s < count; s += kThreads) {
+    SlotState m;
+    load_state(s, m);
+    finish(slot_of(s), meta_s[s], m);
   }
 }
 
-template <int kCap, int kThreads, bool kSplit, bool kServe = false, bool kGather = false, bool kPair = false>
+template <int kCap, int kThreads, bool kServe = false, bool kGather = false, bool kPair = false>
 cudaError_t launch_block_cfg(const StepArgs& args, const int64_t* cta_start, int n_ctas, int n_steps, bool damped,
                              cudaStream_t stream, const ServeCta* serve = nullptr, const int32_t* gmap = nullptr) {
-  const size_t bytes =
-      size_t(damped ? block_rows<true>() : block_rows<false>()) * kCap * sizeof(double) +
-      size_t(kCap) * (sizeof(uint32_t) + sizeof(uint8_t));
+  const size_t bytes = size_t(kBlockRows) * block_row<kCap, kPair>() * sizeof(double) +
+                       size_t(kCap) * (sizeof(uint32_t) + sizeof(uint8_t));
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e != cudaSuccess) return e;
@@ -471,14 +529,14 @@ cudaError_t launch_block_cfg(const StepArgs& args, const int64_t* cta_start, int
   };
   if constexpr (!kServe) {  // serving launches are PositionVerlet
     if (args.n_sub == 4)
-      return damped ? go(rod_block_fp64_kernel<kCap, kThreads, true, kSplit, kServe, kGather, kPair, 1>)
-                    : go(rod_block_fp64_kernel<kCap, kThreads, false, kSplit, kServe, kGather, kPair, 1>);
+      return damped ? go(rod_block_fp64_kernel<kCap, kThreads, true, kServe, kGather, kPair, 1>)
+                    : go(rod_block_fp64_kernel<kCap, kThreads, false, kServe, kGather, kPair, 1>);
     if (args.n_sub == 2)
-      return damped ? go(rod_block_fp64_kernel<kCap, kThreads, true, kSplit, kServe, kGather, kPair, 2>)
-                    : go(rod_block_fp64_kernel<kCap, kThreads, false, kSplit, kServe, kGather, kPair, 2>);
+      return damped ? go(rod_block_fp64_kernel<kCap, kThreads, true, kServe, kGather, kPair, 2>)
+                    : go(rod_block_fp64_kernel<kCap, kThreads, false, kServe, kGather, kPair, 2>);
   }
-  return damped ? go(rod_block_fp64_kernel<kCap, kThreads, true, kSplit, kServe, kGather, kPair>)
-                : go(rod_block_fp64_kernel<kCap, kThreads, false, kSplit, kServe, kGather, kPair>);
+  return damped ? go(rod_block_fp64_kernel<kCap, kThreads, true, kServe, kGather, kPair>)
+                : go(rod_block_fp64_kernel<kCap, kThreads, false, kServe, kGather, kPair>);
 }
 
 }  // namespace
@@ -507,7 +565,7 @@ int block_config_threads(int config) {
 cudaError_t launch_rod_block_fp64_serve(const StepArgs& args, const ServeCta* serve, int n_ctas, int n_steps,
                                         bool damped, cudaStream_t stream) {
   if (n_ctas <= 0 || n_steps <= 0) return cudaSuccess;
-  return launch_block_cfg<520, 512, true, true, false, true>(args, nullptr, n_ctas, n_steps, damped, stream, serve);
+  return launch_block_cfg<520, 512, true, false, true>(args, nullptr, n_ctas, n_steps, damped, stream, serve);
 }
 
 // Rod pairs on gathered CTAs: CTAs 2i and 2i + 1 own the two halves of one
@@ -517,8 +575,8 @@ cudaError_t launch_rod_block_fp64_pairs(const StepArgs& args, const int64_t* cta
                                         int n_ctas, int n_steps, int config, bool damped, cudaStream_t stream) {
   if (n_ctas <= 0 || n_steps <= 0) return cudaSuccess;
   switch (config) {
-    case 0: return launch_block_cfg<520, 512, true, false, true, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
-    case 1: return launch_block_cfg<520, 256, true, false, true, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
+    case 0: return launch_block_cfg<520, 512, false, true, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
+    case 1: return launch_block_cfg<520, 256, false, true, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -529,10 +587,10 @@ cudaError_t launch_rod_block_fp64_gather(const StepArgs& args, const int64_t* ct
                                          int n_ctas, int n_steps, int config, bool damped, cudaStream_t stream) {
   if (n_ctas <= 0 || n_steps <= 0) return cudaSuccess;
   switch (config) {
-    case 0: return launch_block_cfg<520, 512, true, false, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
-    case 1: return launch_block_cfg<520, 256, true, false, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
-    case 2: return launch_block_cfg<264, 256, true, false, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
-    case 3: return launch_block_cfg<320, 320, true, false, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
+    case 0: return launch_block_cfg<520, 512, false, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
+    case 1: return launch_block_cfg<520, 256, false, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
+    case 2: return launch_block_cfg<264, 256, false, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
+    case 3: return launch_block_cfg<320, 320, false, true>(args, cta_start, n_ctas, n_steps, damped, stream, nullptr, gmap);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -1,0 +1,153 @@
+// Cheaper forms of the FP64 rod arithmetic for the resident kernel, each with
+// the result of the plain expression it stands for.
+//
+// The kernel is bound by FP64 issue and by the latency of dependent FP64
+// operations, and a library division or square root is ten or more of them
+// with a branch of its own.  Stiff rods amplify any difference in rounding
+// (two correct evaluations part by 1e-9 in the angular velocities within a
+// few hundred steps), so the forms below are not merely accurate: they round
+// correctly, as IEEE division and square root do.  Each takes a hardware
+// approximation (20 bits or more), one Householder iteration of third order
+// (error e -> O(e^3), below an ulp) and a correction by the exact residual
+// (Markstein's theorem), without branches, so that independent chains
+// interleave.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "rod_math.cuh"
+
+namespace eb {
+
+// an approximation of 1 / d within an ulp, for a normal d whose reciprocal is
+// normal: with e = 1 - d y0, 1 / d = y0 (1 + e + e^2 + O(e^3))
+__device__ __forceinline__ double rcp_near(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// 1 / d from an approximation y of it within a few ulps
+__device__ __forceinline__ double rcp_from(double d, double y) { return fma(fma(-d, y, 1.0), y, y); }
+
+// a / d from y, the rounded 1 / d
+__device__ __forceinline__ double div_from(double a, double d, double y) {
+  const double q = a * y;
+  return fma(fma(-q, d, a), y, q);
+}
+
+// an approximation of 1 / sqrt(z) within an ulp, for a normal z > 0: with
+// e = 1 - z y0^2, 1 / sqrt(z) = y0 (1 + e / 2 + 3 e^2 / 8 + O(e^3))
+__device__ __forceinline__ double rsqrt_near(double z) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(z));
+  const double e = fma(-(z * y), y, 1.0);
+  return fma(y, e * fma(0.375, e, 0.5), y);
+}
+
+// sqrt(z) from y, 1 / sqrt(z) within an ulp
+__device__ __forceinline__ double sqrt_from(double z, double y) {
+  const double g = z * y;
+  return fma(fma(-g, g, z), 0.5 * y, g);
+}
+
+// whether d lies in [2^-400, 2^400]: there the forms above and the products
+// around them stay clear of underflow and overflow; other values (zero, not
+// finite) take the plain operations
+__device__ __forceinline__ bool ordinary(double d) {
+  return static_cast<uint32_t>(__double2hiint(d)) - (623u << 20) < (800u << 20);
+}
+
+// length and reciprocal length from the squared length
+struct Length {
+  double l, il;
+};
+__device__ __forceinline__ Length length_of(double l2) {
+  if (ordinary(l2)) {
+    const double y = rsqrt_near(l2);
+    const double l = sqrt_from(l2, y);
+    return {l, rcp_from(l, y)};
+  }
+  const double l = sqrt(l2);
+  return {l, 1.0 / l};
+}
+
+// The coefficients of so3_update_fast: the rotation is applied to a slot's
+// directors twice a step (the closing half drift of one step and the first of
+// the next have the same angle), so they are formed once.
+struct Rotation {
+  double c, s;      // cos, sin of the angle
+  double u[3];      // guarded axis
+  double au[3];     // (1 - cos) times the axis
+};
+
+__device__ __forceinline__ Rotation rotation(double u0, double u1, double u2) {
+  const double z = u0 * u0 + u1 * u1 + u2 * u2;
+  double theta, r;
+  if (z > 1e-30 && z < 1e30) {
+    // |u| > 1e-15: the guard of 1e-14 changes the sum by at most a factor of
+    // eleven, far from the ends of the range
+    theta = sqrt_from(z, rsqrt_near(z));
+    const double d = theta + 1e-14;
+    r = rcp_from(d, rcp_near(d));
+  } else {
+    theta = sqrt(z);
+    r = 1.0 / (theta + 1e-14);
+  }
+  double s, alpha;
+  if (theta < 0.1) {
+    s = theta * (1.0 + z * (-1.0 / 6.0 + z * (1.0 / 120.0 + z * (-1.0 / 5040.0 +
+                                                           z * (1.0 / 362880.0 - z * (1.0 / 39916800.0))))));
+    alpha = z * (0.5 + z * (-1.0 / 24.0 + z * (1.0 / 720.0 + z * (-1.0 / 40320.0 + z * (1.0 / 3628800.0)))));
+  } else {
+    double c;
+    sincos(theta, &s, &c);
+    alpha = 1.0 - c;
+  }
+  u0 *= r;
+  u1 *= r;
+  u2 *= r;
+  return {1.0 - alpha, s, {u0, u1, u2}, {alpha * u0, alpha * u1, alpha * u2}};
+}
+
+// Q <- R Q; the products are fused as the compiler fuses so3_update_fast
+// (written out, so that every kernel rounds alike)
+__device__ __forceinline__ void rotate(double q[9], const Rotation& R) {
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const double q0 = q[j], q1 = q[3 + j], q2 = q[6 + j];
+    const double com = fma(q2, R.u[2], fma(q0, R.u[0], q1 * R.u[1]));
+    q[j] = fma(R.s, fma(q1, R.u[2], -(q2 * R.u[1])), fma(R.c, q0, R.au[0] * com));
+    q[3 + j] = fma(R.s, fma(q2, R.u[0], -(q0 * R.u[2])), fma(R.au[1], com, R.c * q1));
+    q[6 + j] = fma(R.s, fma(q0, R.u[1], -(q1 * R.u[0])), fma(R.au[2], com, R.c * q2));
+  }
+}
+
+// Curvature as inv_rotate_divide_fast forms it, with the square root and the
+// quotient in the forms above (a 1 - cos(theta) outside (1e-12, 2) takes the
+// plain operations).
+__device__ __forceinline__ Vec3<double> curvature(const double qc[9], const double qn[9], double span) {
+  const double tr = qc[0] * qn[0] + qc[1] * qn[1] + qc[2] * qn[2] + qc[3] * qn[3] + qc[4] * qn[4] +
+                    qc[5] * qn[5] + qc[6] * qn[6] + qc[7] * qn[7] + qc[8] * qn[8];
+  const double cth = 0.5 * tr - (0.5 + 1e-10);
+  const double theta = acos(cth);
+  const double w = (1.0 - cth) * (1.0 + cth);
+  const bool fine = w > 1e-12 && ordinary(span);
+  const double root = fine ? sqrt_from(w, rsqrt_near(w)) : sqrt(w);
+  const double den = (root + cth * 1e-14) * span;
+  const double half = 0.5 * theta;
+  double st;
+  if (fine)
+    st = div_from(half, den, rcp_from(den, rcp_near(den)));
+  else
+    st = half / den;
+  return {st * (-qc[3] * qn[6] - qc[4] * qn[7] - qc[5] * qn[8] + qc[6] * qn[3] + qc[7] * qn[4] +
+                qc[8] * qn[5]),
+          st * (qc[0] * qn[6] + qc[1] * qn[7] + qc[2] * qn[8] - qc[6] * qn[0] - qc[7] * qn[1] -
+                qc[8] * qn[2]),
+          st * (-qc[0] * qn[3] - qc[1] * qn[4] - qc[2] * qn[5] + qc[3] * qn[0] + qc[4] * qn[1] +
+                qc[5] * qn[2])};
+}
+
+}  // namespace eb
