@@ -11,21 +11,22 @@
 //   1. capsule_kernel: capsules and their axis-aligned bounding boxes
 //      (Primitives/detail/CapsulePrimitiveBase.cpp:163-180), and the largest
 //      box extent (block max, one atomic per CTA).
-//   2. cell_kernel + scan + scatter_kernel: a uniform grid with the cell edge
-//      just above the largest extent, hashed into a power-of-two table; every
-//      capsule is filed under the cell of its box's lower corner (a counting
-//      sort by bucket).
-//   3. pairs_kernel<0>: every capsule tests the capsules filed in its 27
-//      neighbouring cells, then every plane, in one pass, writing up to
+//   2. cell_kernel + range_kernel + scatter_kernel: a uniform grid with the
+//      cell edge one or two of the largest extent, a bucket a cell or hashed
+//      into a power-of-two table; every capsule is filed under the cell of its
+//      box's lower corner (a counting sort by bucket).
+//   3. pairs_kernel<0>: every capsule tests the capsules filed in the cells
+//      its box can reach, then every plane, in one pass, writing up to
 //      kFixedPartners partners into its fixed-stride list (sorted) and its
 //      count; a capsule with more partners takes a region of the overflow
 //      lists (one atomic on their total), and pairs_kernel<1> writes its
-//      whole sorted list there.  Two boxes that overlap have lower corners less
-//      than one cell apart on each axis, so the candidate set equals the
+//      whole sorted list there.  A box that overlaps has its lower corner no
+//      further below than the largest extent, so the candidate set equals the
 //      exhaustive search's (Detection/Coarse/ExhaustiveSearch.hpp:322-435,
 //      closed intervals of BoundingBox.hpp:532-540), which the reference's
 //      hash grids reproduce (tests/.../Test_HashGrids.cpp).
-//   4. force_kernel: each capsule evaluates the narrow phase with every
+//   4. force_kernel: each capsule with a partner other than its neighbours on
+//      its rod evaluates the narrow phase with every
 //      partner in ascending id order (RodCapsuleRodCapsule.hpp:70-186,
 //      CapsulePlane.hpp:60-113), the pair always oriented with the smaller id
 //      as the first body, and sums the spring-dashpot loads
@@ -44,7 +45,7 @@
 #include <algorithm>
 
 #include "contact.h"
-#include "rod_math.cuh"
+#include "rod_fast.cuh"
 
 namespace eb {
 namespace {
@@ -64,9 +65,6 @@ constexpr int kThreads = 256;
 // spilled 500 bytes a thread): 0.91 -> 0.82 ms a contact step
 constexpr int kForceThreads = 128;
 constexpr int kForceCtasPerSm = 3;
-constexpr int kScanThreads = 1024;
-constexpr int kScanItems = 4;
-constexpr int kScanBlock = kScanThreads * kScanItems;
 
 __device__ __forceinline__ D3 ld3(const double* p, int64_t S, int64_t s) { return {p[s], p[S + s], p[2 * S + s]}; }
 __device__ __forceinline__ void st3(double* p, int64_t S, int64_t s, D3 a) {
@@ -76,11 +74,24 @@ __device__ __forceinline__ void st3(double* p, int64_t S, int64_t s, D3 a) {
 }
 __device__ __forceinline__ D3 mul3(double k, D3 a) { return {k * a.x, k * a.y, k * a.z}; }
 __device__ __forceinline__ D3 neg3(D3 a) { return {-a.x, -a.y, -a.z}; }
-__device__ __forceinline__ double norm3(D3 a) { return sqrt(a.x * a.x + a.y * a.y + a.z * a.z); }
+// a / b, 1 / b and sqrt(a) in the correctly rounded forms of rod_fast.cuh
+// (their fused operations are written out, so nothing is contracted here)
+__device__ __forceinline__ double reciprocal(double b) { return ordinary(b) ? rcp_from(b, rcp_near(b)) : 1.0 / b; }
+__device__ __forceinline__ double quotient(double a, double b) {
+  return ordinary(b) ? div_from(a, b, rcp_from(b, rcp_near(b))) : a / b;
+}
+__device__ __forceinline__ D3 quotient3(D3 a, double b) {
+  if (!ordinary(b)) return {a.x / b, a.y / b, a.z / b};
+  const double y = rcp_from(b, rcp_near(b));
+  return {div_from(a.x, b, y), div_from(a.y, b, y), div_from(a.z, b, y)};
+}
+__device__ __forceinline__ double root(double a) { return ordinary(a) ? sqrt_from(a, rsqrt_near(a)) : sqrt(a); }
+__device__ __forceinline__ double squared(D3 a) { return a.x * a.x + a.y * a.y + a.z * a.z; }
+__device__ __forceinline__ double norm3(D3 a) { return root(squared(a)); }
 // blaze::normalize: a * (1 / |a|), a zero vector stays zero
 __device__ __forceinline__ D3 normalize3(D3 a) {
-  const double len = norm3(a);
-  const double il = len != 0.0 ? 1.0 / len : 0.0;
+  const Length len = length_of(squared(a));
+  const double il = len.l != 0.0 ? len.il : 0.0;
   return {a.x * il, a.y * il, a.z * il};
 }
 
@@ -103,12 +114,6 @@ __device__ __forceinline__ Capsule load_capsule(const double* cap, int64_t S, in
   return k;
 }
 
-__device__ __forceinline__ bool overlaps(const double alo[3], const double ahi[3], const double blo[3],
-                                         const double bhi[3]) {
-  return !(blo[0] > ahi[0] || blo[1] > ahi[1] || blo[2] > ahi[2] || bhi[0] < alo[0] || bhi[1] < alo[1] ||
-           bhi[2] < alo[2]);
-}
-
 __device__ __forceinline__ uint32_t cell_hash(int32_t cx, int32_t cy, int32_t cz) {
   uint64_t h = static_cast<uint64_t>(static_cast<uint32_t>(cx)) * 0x9E3779B97F4A7C15ull ^
                static_cast<uint64_t>(static_cast<uint32_t>(cy)) * 0xC2B2AE3D27D4EB4Full ^
@@ -119,13 +124,26 @@ __device__ __forceinline__ uint32_t cell_hash(int32_t cx, int32_t cy, int32_t cz
   return static_cast<uint32_t>(h);
 }
 
+// FP32 values as integers of the same order, above zero for every number
+__device__ __forceinline__ uint32_t ordered(float f) {
+  const uint32_t b = __float_as_uint(f);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__device__ __forceinline__ float unordered(uint32_t u) {
+  return __uint_as_float((u & 0x80000000u) ? (u & 0x7fffffffu) : ~u);
+}
+
 // ---- stage 1: capsules and boxes ------------------------------------------
+
+constexpr uint32_t kNotFiled = 0xffffffffu;
 
 __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) {
   const int64_t s = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
   const int64_t S = a.stride;
   double ext = 0.0;
   bool bad = false;
+  // bounds of the lower corners (see ContactGrid): zero takes no part
+  uint32_t top[3] = {0u, 0u, 0u}, bottom[3] = {0u, 0u, 0u};
   if (s < a.n_slots && a.cap_material[s] >= 0) {
     const double* x = a.state + kStX * S;
     const double* v = a.state + kStV * S;
@@ -136,20 +154,45 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
     D3 x0 = {x[s] + c * v[s], x[S + s] + c * v[S + s], x[2 * S + s] + c * v[2 * S + s]};
     D3 x1 = {x[s + 1] + c * v[s + 1], x[S + s + 1] + c * v[S + s + 1], x[2 * S + s + 1] + c * v[2 * S + s + 1]};
     const uint32_t meta = a.meta[s];
+    // the far node of the next element of the rod
+    const bool joint = (meta & kVor) != 0;
+    D3 x2 = x1;
+    if (joint) x2 = {x[s + 2] + c * v[s + 2], x[S + s + 2] + c * v[S + s + 2], x[2 * S + s + 2] + c * v[2 * S + s + 2]};
     if (a.sim_flags & kSimClamp) {
-      // either node of the element may be held by a clamp
+      // any of the nodes may be held by a clamp
       const RodInfo& ri = a.rods[meta >> kRodShift];
       double t[3];
       if (clamp_position(ri, s, t)) x0 = {t[0], t[1], t[2]};
       if (clamp_position(ri, s + 1, t)) x1 = {t[0], t[1], t[2]};
+      if (joint && clamp_position(ri, s + 2, t)) x2 = {t[0], t[1], t[2]};
     }
     const D3 dx = x1 - x0;
-    const double l = norm3(dx);
-    const D3 t = {dx.x / l, dx.y / l, dx.z / l};
-    const double l0 = a.par[kL0 * S + s];
-    const double e = l / l0;
+    const Length len = length_of(squared(dx));
+    const double l = len.l;
+    // Consecutive capsules of a rod share a node, so the narrow phase finds
+    // them no distance apart and no contact.  Its tolerance on the projections
+    // (1e-8 m^2) can only pick another region for elements shorter than a
+    // millimetre or folded back on one another, and the ends only part by
+    // rounding (1e-8 m) far from the origin: such joints are evaluated.
+    {
+      const D3 dn = x2 - x1;
+      const double l2 = dot(dx, dx), n2 = dot(dn, dn), along = dot(dx, dn);
+      a.plain_joint[s] = joint && l2 > 1e-6 && n2 > 1e-6 && l2 < 1e8 && n2 < 1e8 && along > 0.0 &&
+                         along * along > 0.01 * (l2 * n2) && fabs(x1.x) < 1e6 && fabs(x1.y) < 1e6 && fabs(x1.z) < 1e6;
+    }
+    const double l0 = a.par[kL0 * S + s], volume = a.par[kVol * S + s];
+    D3 t;
+    double area;  // volume / (pi l)
+    if (ordinary(l)) {
+      t = {div_from(dx.x, l, len.il), div_from(dx.y, l, len.il), div_from(dx.z, l, len.il)};
+      area = div_from(M_1_PI * volume, l, len.il);
+    } else {
+      t = {dx.x / l, dx.y / l, dx.z / l};
+      area = M_1_PI * volume / l;
+    }
+    const double e = quotient(l, l0);
     const double L = e * l0;
-    const double r = sqrt(M_1_PI * a.par[kVol * S + s] / l);
+    const double r = root(area);
     const D3 cen = {0.5 * (x0.x + x1.x), 0.5 * (x0.y + x1.y), 0.5 * (x0.z + x1.z)};
     // Orthogonal.cpp:32-55 with the tangent as the third row
     const D3 v1 = normalize3(t);
@@ -166,10 +209,13 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
     const D3 va = ld3(v, S, s), vb = ld3(v, S, s + 1);
     const D3 num = mul3(m0, va) + mul3(m1, vb);
     const double den = m0 + m1;
-    const D3 vel = {num.x / den, num.y / den, num.z / den};
+    const D3 vel = quotient3(num, den);
     const D3 om = ld3(w, S, s);
     const D3 ww = {r0.x * om.x + r1.x * om.y + r2.x * om.z, r0.y * om.x + r1.y * om.y + r2.y * om.z,
                    r0.z * om.x + r1.z * om.y + r2.z * om.z};
+    // the narrow phase writes only the capsules it evaluates
+    st3(a.cf, S, s, D3{0.0, 0.0, 0.0});
+    st3(a.ct, S, s, D3{0.0, 0.0, 0.0});
     double* cap = a.cap;
     st3(cap + kCapC * S, S, s, cen);
     cap[kCapL * S + s] = L;
@@ -178,6 +224,9 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
     st3(cap + kCapVel * S, S, s, vel);
     st3(cap + kCapW * S, S, s, ww);
     const double ua[3] = {r2.x, r2.y, r2.z}, ca[3] = {cen.x, cen.y, cen.z};
+    // a capsule whose box is not finite (a diverged state) takes no part: it
+    // would overlap every box
+    bool filed = true;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const double len = fabs(ua[d] * L) * 0.5 + r + kContactThreshold;
@@ -187,13 +236,32 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
       const double xt = hi - lo;
       if (!(xt >= 0.0 && xt < 1e300)) bad = true;  // NaN or infinite box
       else ext = fmax(ext, xt);
+      filed = filed && (xt >= 0.0) && (xt < 1e300) && (fabs(lo) < 1e300);
+      top[d] = ordered(__double2float_ru(lo));
+      bottom[d] = ordered(-__double2float_rd(lo));
+    }
+    a.bucket[s] = filed ? 0u : kNotFiled;
+    if (!filed) {
+      a.pair_count[s] = 0;
+      top[0] = top[1] = top[2] = bottom[0] = bottom[1] = bottom[2] = 0u;
     }
   }
   // block max of the extents, one atomic per CTA (non-negative doubles order
   // like their bit patterns)
   for (int o = 16; o > 0; o >>= 1) ext = fmax(ext, __shfl_xor_sync(0xffffffffu, ext, o));
   __shared__ double wmax[kThreads / 32];
+  __shared__ uint32_t bounds[6];
+  if (threadIdx.x < 6) bounds[threadIdx.x] = 0u;
   if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = ext;
+  __syncthreads();
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const uint32_t t = __reduce_max_sync(0xffffffffu, top[d]), b = __reduce_max_sync(0xffffffffu, bottom[d]);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMax(bounds + d, t);
+      atomicMax(bounds + 3 + d, b);
+    }
+  }
   if (bad) atomicOr(a.status, kStatusContactNonFinite);
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -201,68 +269,202 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
     for (int i = 0; i < kThreads / 32; ++i) m = fmax(m, wmax[i]);
     if (m > 0.0) atomicMax(a.extent_bits, static_cast<unsigned long long>(__double_as_longlong(m)));
   }
+  if (threadIdx.x < 6 && bounds[threadIdx.x])
+    atomicMax(threadIdx.x < 3 ? a.grid->top + threadIdx.x : a.grid->bottom + (threadIdx.x - 3), bounds[threadIdx.x]);
 }
 
 // ---- stage 2: grid cells, counting sort by bucket --------------------------
 
-__device__ __forceinline__ double inverse_cell(const ContactArgs& a) {
-  double h = __longlong_as_double(static_cast<long long>(*a.extent_bits)) * kCellMargin;
-  if (!(h > 0.0)) h = 1.0;
-  return 1.0 / h;
+// Cell edge in units of the largest extent (with its margin): one capsule
+// searches the cells its box can reach, 2.7 an axis for an edge of one
+// (unless its box is as large as the largest, in which case three) and 1.8
+// for an edge of two, whose cells hold eight times the space.  Two wins where
+// the lookups outnumber the records read, which the evaluation before tells
+// (it changes the time only, never the pairs).  The bounds lie a factor apart
+// so that the choice does not alternate.
+__device__ __forceinline__ int32_t choose_edge(const ContactArgs& a) {
+  const int32_t before = a.grid->edge_before;
+  const unsigned long long n = static_cast<unsigned long long>(a.n_caps);
+  const unsigned long long scanned = a.grid->scanned;
+  if (before == 1) return scanned < 8 * n ? 2 : 1;
+  return before == 2 && scanned > 48 * n ? 1 : 2;
+}
+
+__device__ __forceinline__ int32_t cell_of(double x, double inv_edge) {
+  return static_cast<int32_t>(fmin(fmax(floor(x * inv_edge), -kCellClamp), kCellClamp));
+}
+
+// The grid of this evaluation: a bucket a cell when the cells between the
+// lowest and the highest lower corner fit the table, else cells hashed into
+// it.  A bucket a cell needs no hash (four 64-bit multiplications a lookup)
+// and no comparison of cells, and the cells of a row are neighbours in memory.
+__device__ __forceinline__ ContactGrid make_grid(const ContactArgs& a) {
+  ContactGrid g;
+  const double h = __longlong_as_double(static_cast<long long>(*a.extent_bits)) * kCellMargin;
+  g.edge = choose_edge(a);
+  g.reach = h > 0.0 ? h : 1.0;
+  g.inv_edge = 1.0 / (g.edge * g.reach);
+  double total = 1.0;
+  float far = 0.0f;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const bool any = a.grid->top[d] != 0u;
+    const float hi = any ? unordered(a.grid->top[d]) : 0.0f, lo = any ? -unordered(a.grid->bottom[d]) : 0.0f;
+    g.first[d] = cell_of(lo, g.inv_edge);
+    g.last[d] = cell_of(hi, g.inv_edge);
+    total *= static_cast<double>(g.last[d]) - static_cast<double>(g.first[d]) + 1.0;
+    far = fmaxf(far, fmaxf(fabsf(lo), fabsf(hi)));
+  }
+  g.dense = total <= static_cast<double>(a.max_cells);
+  g.row = g.dense ? g.last[0] - g.first[0] + 1 : 0;
+  g.slab = g.dense ? g.row * (g.last[1] - g.first[1] + 1) : 0;
+  // a corner rounded outward lies within 2^-23 of its value (and 1e-44 of
+  // zero), and no corner lies further out than the farthest plus the reach
+  // (beyond FP32's range a NaN: no FP32 comparison decides)
+  const float out = far + static_cast<float>(g.reach);
+  g.sure = out < 1e30f ? out * 1e-6f + 1e-30f : __int_as_float(0x7fffffff);
+  // cells by the FP32 corners, which the records hold, as long as their
+  // rounding (the margin added to the reach) is small against a box
+  const double margin = static_cast<double>(out) * 2.5e-7;
+  g.by_float = margin < 0.125 * g.reach;
+  if (g.by_float) g.reach += margin;
+  return g;
+}
+
+// cell of a lower corner: of its FP32 value rounded down, or of itself
+__device__ __forceinline__ int32_t corner_cell(const ContactGrid& g, double lo) {
+  return cell_of(g.by_float ? static_cast<double>(__double2float_rd(lo)) : lo, g.inv_edge);
+}
+
+// bucket of a cell (in the dense grid: of a cell inside it)
+__device__ __forceinline__ uint32_t bucket_of(const ContactGrid& g, bool dense, uint32_t mask, int32_t cx, int32_t cy,
+                                              int32_t cz) {
+  if (dense)
+    return static_cast<uint32_t>((cz - g.first[2]) * g.slab + (cy - g.first[1]) * g.row + (cx - g.first[0]));
+  return cell_hash(cx, cy, cz) & mask;
 }
 
 __global__ void __launch_bounds__(kThreads) cell_kernel(const ContactArgs a) {
   const int64_t s = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
-  if (s == 0) a.pair_offset[a.n_slots] = 0;  // the pair search's overflow total
-  if (s >= a.n_slots || a.cap_material[s] < 0) return;
-  const int64_t S = a.stride;
-  // a capsule whose box is not finite (a diverged state, already flagged by
-  // the capsule kernel) takes no part: it would overlap every box
-  bool finite = true;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const double lo = a.cap[(kCapLo + d) * S + s], hi = a.cap[(kCapHi + d) * S + s];
-    finite = finite && (hi - lo >= 0.0) && (hi - lo < 1e300) && (fabs(lo) < 1e300);
+  const ContactGrid g = make_grid(a);
+  if (s == 0) {
+    a.pair_offset[a.n_slots] = 0;  // the pair search's overflow total
+    // (none of these is read before the next kernel)
+    a.grid->inv_edge = g.inv_edge;
+    a.grid->reach = g.reach;
+    for (int d = 0; d < 3; ++d) {
+      a.grid->first[d] = g.first[d];
+      a.grid->last[d] = g.last[d];
+    }
+    a.grid->dense = g.dense;
+    a.grid->by_float = g.by_float;
+    a.grid->row = g.row;
+    a.grid->slab = g.slab;
+    a.grid->sure = g.sure;
+    a.grid->edge = g.edge;
+    a.grid->filed = 0;
+    a.grid->live = 0;
   }
-  if (!finite) {
-    a.bucket[s] = 0xffffffffu;
+  if (s >= a.n_slots || a.cap_material[s] < 0 || a.bucket[s] == kNotFiled) return;
+  const int64_t S = a.stride;
+  int32_t c[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) c[d] = corner_cell(g, a.cap[(kCapLo + d) * S + s]);
+  const uint32_t b = bucket_of(g, g.dense, a.table_mask, c[0], c[1], c[2]);
+  if (b >= a.max_cells) {  // cannot happen: the bounds hold every lower corner
+    atomicOr(a.status, kStatusContactIndex);
+    a.bucket[s] = kNotFiled;
     a.pair_count[s] = 0;
     return;
   }
-  const double ih = inverse_cell(a);
-  int32_t c[3];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    double f = floor(a.cap[(kCapLo + d) * S + s] * ih);
-    f = fmin(fmax(f, -kCellClamp), kCellClamp);
-    c[d] = static_cast<int32_t>(f);
-    a.cell[d * S + s] = c[d];
-  }
-  const uint32_t b = cell_hash(c[0], c[1], c[2]) & a.table_mask;
   a.bucket[s] = b;
   // the capsule's rank in its bucket, kept in its pair count until the
   // scatter has filed it (the pair search then writes the count)
   a.pair_count[s] = atomicAdd(a.bucket_count + b, 1);
 }
 
+// The buckets' ranges of entries, in whatever order the CTAs come: a CTA
+// scans the counts of its buckets and takes their entries with one atomic.
+// (A scan of the whole table in bucket order took three launches, 24 us for
+// two million buckets against 8 us; no reader needs the order.)  The counts
+// go back to zero for the next evaluation.
+constexpr int kRangeItems = 8;
+
+__global__ void __launch_bounds__(kThreads) range_kernel(const ContactArgs a) {
+  // buckets in use: the hash table's or the dense grid's cells (max_cells, a
+  // power of two of at least 1024, holds either)
+  const ContactGrid& g = *a.grid;
+  const int64_t used = g.dense ? static_cast<int64_t>(g.slab) * (g.last[2] - g.first[2] + 1)
+                               : static_cast<int64_t>(a.table_mask) + 1;
+  const int64_t first = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) * kRangeItems;
+  if (static_cast<int64_t>(blockIdx.x) * kThreads * kRangeItems >= used) return;
+  const bool on = first < a.max_cells;
+  int32_t n[kRangeItems] = {0, 0, 0, 0, 0, 0, 0, 0};
+  int4* counts = reinterpret_cast<int4*>(a.bucket_count + first);
+  if (on) {
+    const int4 c0 = counts[0], c1 = counts[1];
+    n[0] = c0.x, n[1] = c0.y, n[2] = c0.z, n[3] = c0.w;
+    n[4] = c1.x, n[5] = c1.y, n[6] = c1.z, n[7] = c1.w;
+    counts[0] = counts[1] = make_int4(0, 0, 0, 0);
+  }
+  int32_t sum = 0;
+#pragma unroll
+  for (int i = 0; i < kRangeItems; ++i) sum += n[i];
+  __shared__ int32_t warp_sum[kThreads / 32];
+  __shared__ int32_t base;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  int32_t x = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) warp_sum[wid] = x;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int32_t total = 0;
+    for (int i = 0; i < kThreads / 32; ++i) {
+      const int32_t t = warp_sum[i];
+      warp_sum[i] = total;
+      total += t;
+    }
+    base = total ? atomicAdd(&a.grid->filed, total) : 0;
+  }
+  __syncthreads();
+  if (!on) return;
+  int32_t run = base + warp_sum[wid] + x - sum;
+  int4* out = reinterpret_cast<int4*>(a.bucket_range + first);
+#pragma unroll
+  for (int i = 0; i < kRangeItems; i += 2) {
+    const int32_t mid = run + n[i], end = mid + n[i + 1];
+    out[i / 2] = make_int4(run, mid, mid, end);
+    run = end;
+  }
+}
+
 __global__ void __launch_bounds__(kThreads) scatter_kernel(const ContactArgs a) {
   const int64_t s = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
-  if (s == 0) *a.extent_bits = 0;  // read only by the cell kernel: zero for the next evaluation
+  if (s == 0) {
+    *a.extent_bits = 0;  // read only by the cell kernel: zero for the next evaluation
+    a.grid->edge_before = a.grid->edge;
+    a.grid->scanned = 0;
+    for (int d = 0; d < 3; ++d) a.grid->top[d] = a.grid->bottom[d] = 0u;
+  }
   if (s >= a.n_slots || a.cap_material[s] < 0) return;
   const int64_t S = a.stride;
   const uint32_t b = a.bucket[s];
-  if (b > a.table_mask) return;  // excluded (not finite)
-  const int32_t pos = a.bucket_start[b] + a.pair_count[s];  // the rank the cell kernel took
+  if (b >= a.max_cells) return;  // excluded (not finite)
+  const int32_t pos = a.bucket_range[b].x + a.pair_count[s];  // the rank the cell kernel took
   if (pos < 0 || pos >= a.n_caps) {  // cannot happen with consistent counts; never write out of range
     atomicOr(a.status, kStatusContactIndex);
     return;
   }
-  double* rec = a.sorted_rec + static_cast<int64_t>(kSortedRecDoubles) * pos;
-  *reinterpret_cast<int4*>(rec) = make_int4(a.cell[s], a.cell[S + s], a.cell[2 * S + s], static_cast<int32_t>(s));
-  double2* box = reinterpret_cast<double2*>(rec + 2);
-  box[0] = make_double2(a.cap[kCapLo * S + s], a.cap[(kCapLo + 1) * S + s]);
-  box[1] = make_double2(a.cap[(kCapLo + 2) * S + s], a.cap[kCapHi * S + s]);
-  box[2] = make_double2(a.cap[(kCapHi + 1) * S + s], a.cap[(kCapHi + 2) * S + s]);
+  const double* cap = a.cap;
+  float4* rec = reinterpret_cast<float4*>(a.sorted_rec + pos);
+  rec[0] = make_float4(__double2float_rd(cap[kCapLo * S + s]), __double2float_rd(cap[(kCapLo + 1) * S + s]),
+                       __double2float_rd(cap[(kCapLo + 2) * S + s]), __double2float_ru(cap[kCapHi * S + s]));
+  rec[1] = make_float4(__double2float_ru(cap[(kCapHi + 1) * S + s]), __double2float_ru(cap[(kCapHi + 2) * S + s]),
+                       __int_as_float(static_cast<int32_t>(s)), 0.0f);
 }
 
 // ---- stage 3: candidate pairs ----------------------------------------------
@@ -279,93 +481,143 @@ __device__ __forceinline__ void sort_ids(int32_t* v, int32_t n) {
   }
 }
 
-// The search of one capsule.  kPass 0 (idx: a filed entry, the capsule's
-// cell and box from its record) counts the partners and fills the
-// fixed-stride list; kPass 1 (idx: a slot, leaving at once unless its
-// coalesced count is above kFixedPartners; the cell and box from the
-// slot-major rows the records were written from) writes the overflow list of
-// a capsule with more partners.  The search is bound by dependent round
-// trips to L2: every entry of a neighbouring bucket is one 64-byte record
-// read whole before it is tested (its cell, slot and box were three
-// dependent loads when kept in separate arrays), and the bucket range of the
-// next neighbouring cell is loaded while the current one's entries are
-// scanned.
-template <int kPass>
-__device__ __forceinline__ void search_one(const ContactArgs& a, int32_t n_caps, int64_t idx) {
-  int32_t id, cx, cy, cz;
-  double lo[3], hi[3];
+struct FloatBox {
+  float lo[3], hi[3];
+};
+
+// whether the boxes of slots i and j overlap, from their FP64 corners
+__device__ __forceinline__ bool boxes_overlap(const ContactArgs& a, int64_t i, int64_t j) {
+  const int64_t S = a.stride;
+  bool yes = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double* lo = a.cap + (kCapLo + d) * S;
+    const double* hi = a.cap + (kCapHi + d) * S;
+    yes = yes & !(lo[j] > hi[i]) & !(hi[j] < lo[i]);
+  }
+  return yes;
+}
+
+// The search of one capsule.  kPass 0 (idx: a filed entry) counts the
+// partners and fills the fixed-stride list; kPass 1 (idx: a slot, leaving at
+// once unless its coalesced count is above kFixedPartners) writes the overflow
+// list of a capsule with more partners.
+//
+// A box that overlaps has its lower corner at most `reach` below this box's
+// lower corner (no box is larger) and at or below its upper corner, so the
+// search visits the cells of that range (rounding is monotone, and the margins
+// in `reach` are above it): at most eight with an edge of two.  It is
+// bound by dependent round trips to L2 and by its instructions on diverged
+// lanes, so the ranges of two neighbouring cells are loaded together and their
+// entries scanned in one loop, the next two ranges on their way meanwhile, and
+// an entry is one 32-byte record of FP32 corners.  Rounded outward, they
+// decide every pair but those that overlap by less than `sure`; only these
+// take the FP64 corners.  Against 27 hashed
+// lookups in turn and 64-byte FP64 records, the search of 524,288 capsules
+// went from 160 to 73 us.
+template <int kPass, bool kDense>
+__device__ __forceinline__ uint32_t search_one(const ContactArgs& a, const ContactGrid& g, int32_t n_caps, int64_t idx) {
+  int32_t id;
+  FloatBox me;
   int32_t* out;
   if (kPass == 1) {
     const int64_t s = idx;
     // only filed capsules have a count; the others hold zero
-    if (s >= a.n_slots || a.pair_count[s] <= kFixedPartners) return;
+    if (s >= a.n_slots || a.pair_count[s] <= kFixedPartners) return 0;
     const int64_t total = a.pair_offset[a.n_slots];
     if (total > a.capacity) {
       atomicOr(a.status, kStatusPairOverflow);
       atomicMax(a.required, static_cast<unsigned long long>(total));
-      return;
+      return 0;
     }
     out = a.partners + a.pair_offset[s];  // within [0, capacity)
-    const int64_t S = a.stride;
     id = static_cast<int32_t>(s);
-    cx = a.cell[s];
-    cy = a.cell[S + s];
-    cz = a.cell[2 * S + s];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      lo[d] = a.cap[(kCapLo + d) * S + s];
-      hi[d] = a.cap[(kCapHi + d) * S + s];
+      me.lo[d] = __double2float_rd(a.cap[(kCapLo + d) * a.stride + s]);
+      me.hi[d] = __double2float_ru(a.cap[(kCapHi + d) * a.stride + s]);
     }
   } else {
-    const int32_t e = static_cast<int32_t>(idx);
-    if (e >= n_caps) return;
-    const double* own = a.sorted_rec + static_cast<int64_t>(kSortedRecDoubles) * e;
-    const int4 me = *reinterpret_cast<const int4*>(own);
-    id = me.w;
+    const float4* own = reinterpret_cast<const float4*>(a.sorted_rec + idx);
+    const float4 r0 = own[0], r1 = own[1];
+    me = {{r0.x, r0.y, r0.z}, {r0.w, r1.x, r1.y}};
+    id = __float_as_int(r1.z);
     out = a.fixed + static_cast<int64_t>(id) * kFixedPartners;
-    cx = me.x;
-    cy = me.y;
-    cz = me.z;
-    const double2* ob = reinterpret_cast<const double2*>(own + 2);
-    const double2 o0 = ob[0], o1 = ob[1], o2 = ob[2];
-    lo[0] = o0.x;
-    lo[1] = o0.y;
-    lo[2] = o1.x;
-    hi[0] = o1.y;
-    hi[1] = o2.x;
-    hi[2] = o2.y;
+  }
+  // joints with the neighbours on the rod that the narrow phase may skip
+  // (slot id - 1 of a rod's first element is a node slot, which holds zero)
+  const int32_t next = kPass == 0 && a.plain_joint[id] ? id + 1 : -1;
+  const int32_t prev = kPass == 0 && id > 0 && a.plain_joint[id - 1] ? id - 1 : -1;
+  int32_t c0[3], c1[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double lo = g.by_float ? me.lo[d] : a.cap[(kCapLo + d) * a.stride + id];
+    const double hi = g.by_float ? me.hi[d] : a.cap[(kCapHi + d) * a.stride + id];
+    c0[d] = max(cell_of(lo - g.reach, g.inv_edge), g.first[d]);
+    c1[d] = min(cell_of(hi, g.inv_edge), g.last[d]);
   }
   int32_t cnt = 0;
-  // neighbour cell c: dx = c % 3 - 1 fastest, then dy, then dz
-  uint32_t b = cell_hash(cx - 1, cy - 1, cz - 1) & a.table_mask;
-  int32_t next0 = a.bucket_start[b], next1 = a.bucket_start[b + 1];
-  for (int c = 0; c < 27; ++c) {
-    const int32_t nx = cx + c % 3 - 1, ny = cy + (c / 3) % 3 - 1, nz = cz + c / 9 - 1;
-    const int32_t k0 = max(next0, 0), k1 = min(next1, n_caps);
-    if (c + 1 < 27) {
-      b = cell_hash(cx + (c + 1) % 3 - 1, cy + ((c + 1) / 3) % 3 - 1, cz + (c + 1) / 9 - 1) & a.table_mask;
-      next0 = a.bucket_start[b];
-      next1 = a.bucket_start[b + 1];
+  uint32_t scanned = 0;
+  bool live = false;
+  int32_t cx = c0[0], cy = c0[1], cz = c0[2];
+  bool more = c0[0] <= c1[0] && c0[1] <= c1[1] && c0[2] <= c1[2];
+  // the ranges of cells cx and cx + 1 of the row
+  int2 ra = make_int2(0, 0), rb = make_int2(0, 0);
+  auto fetch = [&]() {
+    ra = a.bucket_range[bucket_of(g, kDense, a.table_mask, cx, cy, cz)];
+    rb = cx < c1[0] ? a.bucket_range[bucket_of(g, kDense, a.table_mask, cx + 1, cy, cz)] : make_int2(0, 0);
+  };
+  if (more) fetch();
+  while (more) {
+    const int32_t hx = cx, hy = cy, hz = cz;
+    const int32_t a0 = max(ra.x, 0), na = max(min(ra.y, n_caps) - a0, 0);
+    const int32_t b0 = max(rb.x, 0), n = na + max(min(rb.y, n_caps) - b0, 0);
+    cx += 2;
+    if (cx > c1[0]) {
+      cx = c0[0];
+      if (++cy > c1[1]) {
+        cy = c0[1];
+        ++cz;
+      }
     }
-    for (int32_t k = k0; k < k1; ++k) {
-      const double* r = a.sorted_rec + static_cast<int64_t>(kSortedRecDoubles) * k;
-      const int4 h = *reinterpret_cast<const int4*>(r);
-      const double2* rb = reinterpret_cast<const double2*>(r + 2);
-      const double2 b0 = rb[0], b1 = rb[1], b2 = rb[2];
-      // every part of the record is used whatever the cell, so all four
-      // loads issue together
-      const bool in_cell = (h.x == nx) & (h.y == ny) & (h.z == nz) & (h.w != id);
-      const bool apart = (b0.x > hi[0]) | (b0.y > hi[1]) | (b1.x > hi[2]) | (b1.y < lo[0]) | (b2.x < lo[1]) |
-                         (b2.y < lo[2]);
-      if (!in_cell || apart) continue;
-      if (kPass == 1 || cnt < kFixedPartners) out[cnt] = h.w;
+    more = cz <= c1[2];
+    if (more) fetch();
+    scanned += n;
+    for (int32_t k = 0; k < n; ++k) {
+      const float4* r = reinterpret_cast<const float4*>(a.sorted_rec + (k < na ? a0 + k : b0 + (k - na)));
+      const float4 e0 = r[0], e1 = r[1];
+      const int32_t o = __float_as_int(e1.z);
+      // how far the boxes overlap, the least of the axes and sides
+      const float by = fminf(fminf(fminf(me.hi[0] - e0.x, me.hi[1] - e0.y), fminf(me.hi[2] - e0.z, e0.w - me.lo[0])),
+                             fminf(e1.x - me.lo[1], e1.y - me.lo[2]));
+      if (by < 0.0f || o == id) continue;
+      if (!(by >= g.sure) && !boxes_overlap(a, id, o)) continue;
+      if (!kDense) {  // the entry may be of another cell of this bucket
+        const double* lo = a.cap + kCapLo * a.stride + o;
+        const int64_t S = a.stride;
+        const double x = g.by_float ? e0.x : lo[0], y = g.by_float ? e0.y : lo[S], z = g.by_float ? e0.z : lo[2 * S];
+        if (cell_of(x, g.inv_edge) != (k < na ? hx : hx + 1) || cell_of(y, g.inv_edge) != hy ||
+            cell_of(z, g.inv_edge) != hz)
+          continue;
+      }
+      if (kPass == 1 || cnt < kFixedPartners) out[cnt] = o;
       ++cnt;
+      live = live || (o != next && o != prev);
     }
   }
   for (int32_t p = 0; p < a.n_planes; ++p) {
-    if (!overlaps(lo, hi, a.planes[p].lo, a.planes[p].hi)) continue;
+    const ContactPlane& P = a.planes[p];
+    bool yes = true;
+#pragma unroll
+    for (int d = 0; d < 3; ++d) yes = yes & !(P.lo[d] > me.hi[d]) & !(P.hi[d] < me.lo[d]);
+    if (!yes) continue;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+      yes = yes & !(P.lo[d] > a.cap[(kCapHi + d) * a.stride + id]) & !(P.hi[d] < a.cap[(kCapLo + d) * a.stride + id]);
+    if (!yes) continue;
     if (kPass == 1 || cnt < kFixedPartners) out[cnt] = static_cast<int32_t>(a.n_slots) + p;
     ++cnt;
+    live = true;
   }
   if (kPass == 0) {
     a.pair_count[id] = cnt;
@@ -375,110 +627,46 @@ __device__ __forceinline__ void search_one(const ContactArgs& a, int32_t n_caps,
       a.pair_offset[id] = static_cast<int64_t>(atomicAdd(
           reinterpret_cast<unsigned long long*>(a.pair_offset + a.n_slots), static_cast<unsigned long long>(cnt)));
     if (cnt <= kFixedPartners) sort_ids(out, cnt);  // ascending partner order
+    // the narrow phase's list, one atomic for the lanes that come here together
+    if (live) {
+      const unsigned lanes = __activemask();
+      const int lane = threadIdx.x & 31, first = __ffs(lanes) - 1;
+      int32_t base = 0;
+      if (lane == first) base = atomicAdd(&a.grid->live, __popc(lanes));
+      base = __shfl_sync(lanes, base, first);
+      a.live[base + __popc(lanes & ((1u << lane) - 1u))] = id;  // one entry a filed capsule: below n_caps
+    }
   } else {
     sort_ids(out, cnt);
   }
+  return scanned;
 }
 
 // a grid of resident CTAs whose threads step through the entries (pass 0) or
-// slots (pass 1), as the narrow phase does
+// slots (pass 1, which leaves at once when no capsule overflowed), as the
+// narrow phase does
 template <int kPass>
-__global__ void __launch_bounds__(kThreads) pairs_kernel(const ContactArgs a, int32_t n_caps_max) {
+__global__ void __launch_bounds__(kThreads, 4) pairs_kernel(const ContactArgs a) {
+  if (kPass == 1 && a.pair_offset[a.n_slots] == 0) return;
   // entries filed this evaluation (the capsules with finite boxes)
-  const int32_t n_caps = min(a.bucket_start[a.table_mask + 1], n_caps_max);
+  const int32_t n_caps = min(a.grid->filed, a.n_caps);
+  // (read from shared memory where it is used: in registers it costs the
+  // search two of five CTAs an SM)
+  __shared__ ContactGrid g;
+  if (threadIdx.x == 0) g = *a.grid;
+  __syncthreads();
   const int64_t n = kPass == 1 ? a.n_slots : n_caps;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kThreads;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x; i < n; i += stride)
-    search_one<kPass>(a, n_caps, i);
-}
-
-// ---- exclusive scan of int32 counts (out[n] = total), accumulated in Acc ----
-
-template <typename Acc>
-__device__ __forceinline__ Acc block_exclusive_scan(Acc v, Acc* total) {
-  __shared__ Acc warp_sums[kScanThreads / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  Acc x = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const Acc y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+  uint32_t scanned = 0;
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  if (g.dense)
+    for (int64_t i = first; i < n; i += stride) scanned += search_one<kPass, true>(a, g, n_caps, i);
+  else
+    for (int64_t i = first; i < n; i += stride) scanned += search_one<kPass, false>(a, g, n_caps, i);
+  if (kPass == 0) {
+    scanned = __reduce_add_sync(0xffffffffu, scanned);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&a.grid->scanned, static_cast<unsigned long long>(scanned));
   }
-  if (lane == 31) warp_sums[wid] = x;
-  __syncthreads();
-  if (wid == 0) {
-    Acc ws = warp_sums[lane];
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const Acc y = __shfl_up_sync(0xffffffffu, ws, o);
-      if (lane >= o) ws += y;
-    }
-    warp_sums[lane] = ws;
-  }
-  __syncthreads();
-  const Acc prefix = (wid > 0 ? warp_sums[wid - 1] : Acc(0)) + x - v;
-  *total = warp_sums[kScanThreads / 32 - 1];
-  __syncthreads();
-  return prefix;
-}
-
-template <typename Acc>
-__global__ void __launch_bounds__(kScanThreads) scan_partial(int32_t* in, Acc* out, int64_t n, Acc* block_sums,
-                                                             bool zero_in) {
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanBlock + static_cast<int64_t>(threadIdx.x) * kScanItems;
-  Acc v[kScanItems];
-  Acc sum = 0;
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    v[i] = base + i < n ? static_cast<Acc>(in[base + i]) : Acc(0);
-    sum += v[i];
-  }
-  Acc total;
-  Acc run = block_exclusive_scan<Acc>(sum, &total);
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    if (base + i < n) {
-      out[base + i] = run;
-      if (zero_in) in[base + i] = 0;
-    }
-    run += v[i];
-  }
-  if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-template <typename Acc>
-__global__ void __launch_bounds__(kScanThreads) scan_top(Acc* block_sums, int64_t nb, Acc* out, int64_t n) {
-  Acc carry = 0;
-  for (int64_t base = 0; base < nb; base += kScanThreads) {
-    const int64_t i = base + threadIdx.x;
-    const Acc v = i < nb ? block_sums[i] : Acc(0);
-    Acc total;
-    const Acc pre = block_exclusive_scan<Acc>(v, &total);
-    if (i < nb) block_sums[i] = carry + pre;
-    carry += total;
-  }
-  if (threadIdx.x == 0) out[n] = carry;
-}
-
-template <typename Acc>
-__global__ void __launch_bounds__(kScanThreads) scan_add(Acc* out, int64_t n, const Acc* block_sums) {
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanBlock + static_cast<int64_t>(threadIdx.x) * kScanItems;
-  const Acc add = block_sums[blockIdx.x];
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i)
-    if (base + i < n) out[base + i] += add;
-}
-
-template <typename Acc>
-cudaError_t exclusive_scan(int32_t* in, Acc* out, int64_t n, Acc* block_sums, bool zero_in, cudaStream_t stream,
-                           int64_t* launches) {
-  const int64_t nb = (n + kScanBlock - 1) / kScanBlock;
-  if (nb > 0)
-    scan_partial<Acc><<<static_cast<unsigned>(nb), kScanThreads, 0, stream>>>(in, out, n, block_sums, zero_in);
-  scan_top<Acc><<<1, kScanThreads, 0, stream>>>(block_sums, nb, out, n);
-  if (nb > 0) scan_add<Acc><<<static_cast<unsigned>(nb), kScanThreads, 0, stream>>>(out, n, block_sums);
-  *launches += nb > 0 ? 3 : 1;
-  return cudaGetLastError();
 }
 
 // ---- stage 4: narrow phase and spring-dashpot loads ------------------------
@@ -520,7 +708,7 @@ __device__ void closest_segment_points(D3 a1, D3 a2, D3 b1, D3 b2, D3& cp1, D3& 
   }
   const double la = dot(a1a2, a1a2);
   if (da1 >= -kParallelThreshold && da3 <= kParallelThreshold) {
-    const D3 k = mul3(da1 / la, a1a2);
+    const D3 k = mul3(quotient(da1, la), a1a2);
     const D3 n = a1b1 - k;
     if (dot(b1b2, n) >= -kParallelThreshold) {
       cp1 = a1 + k;
@@ -529,7 +717,7 @@ __device__ void closest_segment_points(D3 a1, D3 a2, D3 b1, D3 b2, D3& cp1, D3& 
     }
   }
   if (da2 >= -kParallelThreshold && da4 <= kParallelThreshold) {
-    const D3 k = mul3(da2 / la, a1a2);
+    const D3 k = mul3(quotient(da2, la), a1a2);
     const D3 n = a1b2 - k;
     if (dot(b1b2, n) <= kParallelThreshold) {
       cp1 = a1 + k;
@@ -539,7 +727,7 @@ __device__ void closest_segment_points(D3 a1, D3 a2, D3 b1, D3 b2, D3& cp1, D3& 
   }
   const double lb = dot(b1b2, b1b2);
   if (db1 <= kParallelThreshold && db2 >= -kParallelThreshold) {
-    const D3 k = mul3(-db1 / lb, b1b2);
+    const D3 k = mul3(quotient(-db1, lb), b1b2);
     const D3 n = neg3(a1b1) - k;
     if (dot(a1a2, n) >= -kParallelThreshold) {
       cp1 = a1;
@@ -548,7 +736,7 @@ __device__ void closest_segment_points(D3 a1, D3 a2, D3 b1, D3 b2, D3& cp1, D3& 
     }
   }
   if (db3 <= kParallelThreshold && db4 >= -kParallelThreshold) {
-    const D3 k = mul3(-db3 / lb, b1b2);
+    const D3 k = mul3(quotient(-db3, lb), b1b2);
     const D3 n = neg3(a2b1) - k;
     if (dot(a1a2, n) <= kParallelThreshold) {
       cp1 = a2;
@@ -558,7 +746,7 @@ __device__ void closest_segment_points(D3 a1, D3 a2, D3 b1, D3 b2, D3& cp1, D3& 
   }
   const double sc = dot(a1a2, b1b2);
   double div = la * lb - sc * sc;
-  div = 1.0 / div;
+  div = reciprocal(div);
   const double sp = (lb * da1 - sc * db1) * div;
   const double tp = (sc * da1 - la * db1) * div;
   cp1 = a1 + mul3(sp, a1a2);
@@ -660,6 +848,7 @@ __device__ __forceinline__ void force_one(const ContactArgs& a, int64_t s) {
     ContactPoint pts[2];
     for (int32_t k = 0; k < cnt; ++k) {
       const int64_t o = list[k];
+      if (o == s + 1 ? a.plain_joint[s] : (o == s - 1 && a.plain_joint[o])) continue;  // no contact (capsule_kernel)
       if (o >= 0 && o < a.n_slots) {
         const int32_t om = a.cap_material[o];
         if (om < 0) continue;
@@ -707,45 +896,39 @@ __device__ __forceinline__ void force_one(const ContactArgs& a, int64_t s) {
 // (with the pair search done the same way: 0.691 -> 0.679 ms a contact step)
 __global__ void __launch_bounds__(kForceThreads, kForceCtasPerSm) force_kernel(const ContactArgs a) {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kForceThreads;
-  for (int64_t s = static_cast<int64_t>(blockIdx.x) * kForceThreads + threadIdx.x; s < a.n_slots; s += stride)
-    force_one(a, s);
+  const int64_t n = min(a.grid->live, a.n_caps);
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kForceThreads + threadIdx.x; i < n; i += stride)
+    force_one(a, a.live[i]);
 }
 
 }  // namespace
-
-int64_t contact_scan_blocks(int64_t n) { return (n + kScanBlock - 1) / kScanBlock + 1; }
 
 cudaError_t launch_contact(const ContactArgs& a, cudaStream_t stream, int64_t* launches) {
   if (a.n_slots <= 0) return cudaSuccess;
   const unsigned gs = static_cast<unsigned>((a.n_slots + kThreads - 1) / kThreads);
   // the largest box extent and the bucket counts are zero here: allocated
   // zeroed, the extent set back to zero by the scatter once the cell kernel
-  // has used it, and each count by the scan as it reads it; the cell kernel
-  // zeroes the overflow lists' running total
-  cudaError_t e = cudaSuccess;
-  const int64_t table = static_cast<int64_t>(a.table_mask) + 1;
+  // has used it, and each count by the range kernel as it reads it; the cell
+  // kernel zeroes the running totals
+  const int64_t table = a.max_cells;
   capsule_kernel<<<gs, kThreads, 0, stream>>>(a);
   cell_kernel<<<gs, kThreads, 0, stream>>>(a);
-  *launches += 2;
-  e = exclusive_scan<int32_t>(a.bucket_count, a.bucket_start, table, reinterpret_cast<int32_t*>(a.scan_blocks), true,
-                             stream, launches);
-  if (e != cudaSuccess) return e;
+  range_kernel<<<static_cast<unsigned>((table + kThreads * kRangeItems - 1) / (kThreads * kRangeItems)), kThreads, 0,
+                 stream>>>(a);
   scatter_kernel<<<gs, kThreads, 0, stream>>>(a);
+  *launches += 4;
   const unsigned ge = static_cast<unsigned>((a.n_caps + kThreads - 1) / kThreads);
-  int pdev = 0, psms = 148;
-  if (cudaGetDevice(&pdev) == cudaSuccess) cudaDeviceGetAttribute(&psms, cudaDevAttrMultiProcessorCount, pdev);
-  int pper = 1;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pper, pairs_kernel<0>, kThreads, 0);
-  const unsigned pblocks = static_cast<unsigned>(std::min<int64_t>(ge, static_cast<int64_t>(psms) * std::max(pper, 1)));
-  if (ge > 0) pairs_kernel<0><<<pblocks, kThreads, 0, stream>>>(a, a.n_caps);
-  *launches += 2;
-  pairs_kernel<1><<<gs, kThreads, 0, stream>>>(a, a.n_caps);
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t fblocks = std::min<int64_t>((a.n_slots + kForceThreads - 1) / kForceThreads,
+  int pper = 1;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&pper, pairs_kernel<0>, kThreads, 0);
+  const unsigned pblocks = static_cast<unsigned>(std::min<int64_t>(ge, static_cast<int64_t>(sms) * std::max(pper, 1)));
+  if (ge > 0) pairs_kernel<0><<<pblocks, kThreads, 0, stream>>>(a);
+  pairs_kernel<1><<<static_cast<unsigned>(std::min<int64_t>(gs, 4 * static_cast<int64_t>(sms))), kThreads, 0, stream>>>(a);
+  const int64_t fblocks = std::min<int64_t>((a.n_caps + kForceThreads - 1) / kForceThreads,
                                             static_cast<int64_t>(sms) * kForceCtasPerSm);
-  force_kernel<<<static_cast<unsigned>(fblocks), kForceThreads, 0, stream>>>(a);
-  *launches += 2;
+  if (fblocks > 0) force_kernel<<<static_cast<unsigned>(fblocks), kForceThreads, 0, stream>>>(a);
+  *launches += 3;
   return cudaGetLastError();
 }
 

@@ -23,7 +23,13 @@ enum CapsuleRow : int {
   kCapRows = 20
 };
 
-constexpr int kSortedRecDoubles = 8;
+// a capsule filed in the grid: its box rounded outward to FP32 and its slot,
+// one 32-byte sector
+struct alignas(32) ContactRecord {
+  float lo[3], hi[3];
+  int32_t slot;
+  int32_t pad;
+};
 
 // partners a capsule keeps in its fixed-stride list; a capsule with more
 // (a pile-up) gets its whole list in the overflow lists instead
@@ -44,6 +50,26 @@ struct ContactPair {
   double k, cn, ct, mu_s, mu_d;
 };
 
+// the grid of one evaluation and what chooses it (device memory, zeroed once)
+struct ContactGrid {
+  double inv_edge;             // 1 / cell edge of this evaluation
+  double reach;                // largest box extent with its margin: how far below a box's lower
+                               // corner the lower corner of an overlapping box may lie
+  int32_t first[3], last[3];   // lowest and highest cell of a lower corner, each axis
+  int32_t dense;               // 1: a bucket a cell (the cells fit the table), 0: hashed
+  int32_t by_float;            // 1: a capsule's cell is that of its FP32 lower corner, 0: of the FP64 one
+  int32_t row, slab;           // dense: cells a row (x) and a slab (x, y)
+  float sure;                  // FP32 boxes that overlap by this much overlap
+  int32_t edge;                // cell edge of this evaluation in units of reach (1 or 2)
+  int32_t edge_before;         // of the evaluation before (0: none yet)
+  unsigned long long scanned;  // records the evaluation before read in its search
+  int32_t filed;               // capsules filed in the grid
+  int32_t live;                // capsules in the list of those the narrow phase evaluates
+  // bounds of the boxes' lower corners, rounded outward to FP32: the largest
+  // and the negated smallest as order-preserving integers (zero: none yet)
+  uint32_t top[3], bottom[3];
+};
+
 struct ContactArgs {
   int64_t stride;
   int64_t n_slots;
@@ -56,17 +82,20 @@ struct ContactArgs {
   uint32_t sim_flags;
   double* cap;                       // kCapRows x stride
   unsigned long long* extent_bits;   // largest box extent (bits of a non-negative double)
-  int32_t* cell;                     // 3 x stride
-  uint32_t* bucket;                  // stride
+  uint32_t* bucket;                  // stride; all ones: not filed (no finite box)
   uint32_t table_mask;               // hash table size - 1 (power of two)
-  int32_t* bucket_count;             // table size (zero between steps)
-  int32_t* bucket_start;             // table size + 1
-  // the capsules grouped by bucket, one 64-byte record an entry: cell
-  // (3 x int32) and slot (int32) in the first 16 bytes, then the box's lower
-  // and upper corners (6 doubles)
-  double* sorted_rec;                // kSortedRecDoubles per entry
+  uint32_t max_cells;                // buckets of the tables below: cells a dense grid may have (at least
+                                     // the hash table's size)
+  int32_t* bucket_count;             // max_cells (zero between steps)
+  int2* bucket_range;                // max_cells: a bucket's first entry and the one past its last
+  ContactGrid* grid;
+  ContactRecord* sorted_rec;         // n_caps: the capsules grouped by bucket
   int32_t* pair_count;               // stride (zero outside capsules): partners per capsule (between
                                      // the cell kernel and the scatter: the capsule's rank in its bucket)
+  // per element slot: 1 if its capsule and the next one of its rod meet end to
+  // end and plainly bent, so that the narrow phase finds no contact between them
+  uint8_t* plain_joint;
+  int32_t* live;                     // n_caps: the capsules with any other partner
   int32_t* fixed;                    // kFixedPartners x stride: partner lists of up to kFixedPartners
   int64_t* pair_offset;              // n_slots + 1: a capsule's overflow list (if it has more than
                                      // kFixedPartners partners); [n_slots] their total
@@ -80,15 +109,11 @@ struct ContactArgs {
   double* cf;                        // 3 x stride, capsule force (lab frame)
   double* ct;                        // 3 x stride, capsule torque (lab frame)
   int32_t n_caps;                    // number of capsules (fixed at finalize)
-  int64_t* scan_blocks;              // block sums of the scans
   uint32_t* status;
 };
 
 // one whole contact evaluation (capsules, candidate pairs, contact loads)
 // for the state a.state at the start of a step; launches counted into *launches
 cudaError_t launch_contact(const ContactArgs& a, cudaStream_t stream, int64_t* launches);
-
-// scratch sizes of launch_contact's scans
-int64_t contact_scan_blocks(int64_t n);
 
 }  // namespace eb

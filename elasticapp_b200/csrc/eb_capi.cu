@@ -125,15 +125,18 @@ struct ContactDevice {
   bool on = false;
   int32_t n_caps = 0;
   uint32_t table_mask = 0;
+  uint32_t max_cells = 0;
   int64_t capacity = 0;
   double* cap = nullptr;
   int32_t* cap_material = nullptr;
   unsigned long long* extent = nullptr;
-  int32_t* cell = nullptr;
   uint32_t* bucket = nullptr;
   int32_t* bucket_count = nullptr;
-  int32_t* bucket_start = nullptr;
-  double* sorted_rec = nullptr;
+  int2* bucket_range = nullptr;
+  eb::ContactGrid* grid = nullptr;
+  uint8_t* plain_joint = nullptr;
+  int32_t* live = nullptr;
+  eb::ContactRecord* sorted_rec = nullptr;
   int32_t* pair_count = nullptr;
   int32_t* fixed = nullptr;
   int64_t* pair_offset = nullptr;
@@ -142,7 +145,6 @@ struct ContactDevice {
   eb::ContactPlane* planes = nullptr;
   eb::ContactPair* pair_table = nullptr;
   double* loads = nullptr;  // 6 x stride: force rows 0-2, torque rows 3-5
-  int64_t* scan_blocks = nullptr;
   double* backup = nullptr;  // state at the start of a step chunk
   bool evaluated = false;
 };
@@ -444,10 +446,11 @@ void host_free(eb_sim* s) {
       g = nullptr;
     }
   ContactDevice& c = s->contact;
-  void* cptrs[] = {c.cap, c.cap_material, c.extent, c.cell, c.bucket, c.bucket_count, c.bucket_start,
+  void* cptrs[] = {c.cap, c.cap_material, c.extent, c.bucket, c.bucket_count, c.bucket_range,
+                   c.grid, c.plain_joint, c.live,
                    c.sorted_rec, c.pair_count, c.fixed, c.pair_offset,
                    c.partners,
-                   c.required, c.planes, c.pair_table, c.loads, c.scan_blocks, c.backup};
+                   c.required, c.planes, c.pair_table, c.loads, c.backup};
   for (void* p : cptrs)
     if (p) cudaFree(p);
   c = ContactDevice{};
@@ -553,6 +556,7 @@ eb_status setup_contact(eb_sim* s) {
   // (contact step 0.646 -> 0.633 ms against two a capsule; eight: 0.645 ms)
   while (table < 4 * n_caps) table <<= 1;
   c.table_mask = static_cast<uint32_t>(table - 1);
+  c.max_cells = static_cast<uint32_t>(2 * table);  // a dense grid of up to eight cells a capsule
   c.capacity = std::max<int64_t>(int64_t(1) << 16, 4 * n_caps);  // overflow lists only
   const size_t nm = s->materials.size();
   std::vector<eb::ContactPair> pairs(nm * nm);
@@ -565,7 +569,6 @@ eb_status setup_contact(eb_sim* s) {
                            1.0 / (1.0 / a.tangential_damping + 1.0 / b.tangential_damping),
                            a.static_friction + b.static_friction, a.dynamic_friction + b.dynamic_friction};
     }
-  const int64_t scan_blocks = eb::contact_scan_blocks(std::max<int64_t>(table, s->n_slots + 1));
   cudaError_t e = cudaSuccess;
   auto alloc = [&](auto** p, size_t bytes) {
     if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(p), bytes);
@@ -574,11 +577,13 @@ eb_status setup_contact(eb_sim* s) {
   alloc(&c.cap, static_cast<size_t>(eb::kCapRows * S) * sizeof(double));
   alloc(&c.cap_material, static_cast<size_t>(S) * sizeof(int32_t));
   alloc(&c.extent, sizeof(unsigned long long));
-  alloc(&c.cell, static_cast<size_t>(3 * S) * sizeof(int32_t));
   alloc(&c.bucket, static_cast<size_t>(S) * sizeof(uint32_t));
-  alloc(&c.bucket_count, static_cast<size_t>(table) * sizeof(int32_t));
-  alloc(&c.bucket_start, static_cast<size_t>(table + 1) * sizeof(int32_t));
-  alloc(&c.sorted_rec, static_cast<size_t>(eb::kSortedRecDoubles * n_caps) * sizeof(double));
+  alloc(&c.bucket_count, static_cast<size_t>(c.max_cells) * sizeof(int32_t));
+  alloc(&c.bucket_range, static_cast<size_t>(c.max_cells) * sizeof(int2));
+  alloc(&c.grid, sizeof(eb::ContactGrid));
+  alloc(&c.plain_joint, static_cast<size_t>(S));
+  alloc(&c.live, static_cast<size_t>(n_caps) * sizeof(int32_t));
+  alloc(&c.sorted_rec, static_cast<size_t>(n_caps) * sizeof(eb::ContactRecord));
   alloc(&c.pair_count, static_cast<size_t>(S) * sizeof(int32_t));
   alloc(&c.fixed, static_cast<size_t>(S) * eb::kFixedPartners * sizeof(int32_t));
   alloc(&c.pair_offset, static_cast<size_t>(s->n_slots + 1) * sizeof(int64_t));
@@ -587,7 +592,6 @@ eb_status setup_contact(eb_sim* s) {
   alloc(&c.planes, std::max<size_t>(1, s->planes.size()) * sizeof(eb::ContactPlane));
   alloc(&c.pair_table, std::max<size_t>(1, pairs.size()) * sizeof(eb::ContactPair));
   alloc(&c.loads, static_cast<size_t>(6 * S) * sizeof(double));
-  alloc(&c.scan_blocks, static_cast<size_t>(scan_blocks) * sizeof(int64_t));
   alloc(&c.backup, static_cast<size_t>(eb::kStateFields * S) * sizeof(double));
   if (e != cudaSuccess)
     return fail(e == cudaErrorMemoryAllocation ? EB_ERR_OUT_OF_MEMORY : EB_ERR_CUDA,
@@ -1722,11 +1726,14 @@ eb::ContactArgs contact_args(eb_sim* s, double dt) {
   a.sim_flags = s->sim_flags;
   a.cap = c.cap;
   a.extent_bits = c.extent;
-  a.cell = c.cell;
   a.bucket = c.bucket;
   a.table_mask = c.table_mask;
+  a.max_cells = c.max_cells;
   a.bucket_count = c.bucket_count;
-  a.bucket_start = c.bucket_start;
+  a.bucket_range = c.bucket_range;
+  a.grid = c.grid;
+  a.plain_joint = c.plain_joint;
+  a.live = c.live;
   a.sorted_rec = c.sorted_rec;
   a.pair_count = c.pair_count;
   a.fixed = c.fixed;
@@ -1741,7 +1748,6 @@ eb::ContactArgs contact_args(eb_sim* s, double dt) {
   a.cf = c.loads;
   a.ct = c.loads + 3 * s->stride;
   a.n_caps = c.n_caps;
-  a.scan_blocks = c.scan_blocks;
   a.status = s->d_status;
   return a;
 }

@@ -28,8 +28,14 @@ __device__ __forceinline__ double rcp_near(double d) {
   return fma(y, fma(e, e, e), y);
 }
 
-// 1 / d from an approximation y of it within a few ulps
-__device__ __forceinline__ double rcp_from(double d, double y) { return fma(fma(-d, y, 1.0), y, y); }
+// 1 / d from an approximation y of it within a few ulps.  The correction
+// multiplies the residual by y or the number after it: for a d just below a
+// power of two (a dilatation of 1 - 2^-53, say) the corrected value is within
+// 2^-105 of a tie, which the larger factor breaks to the right side; for any
+// other d the two round alike.
+__device__ __forceinline__ double rcp_from(double d, double y) {
+  return fma(fma(-d, y, 1.0), __longlong_as_double(__double_as_longlong(y) | 1ll), y);
+}
 
 // a / d from y, the rounded 1 / d
 __device__ __forceinline__ double div_from(double a, double d, double y) {
