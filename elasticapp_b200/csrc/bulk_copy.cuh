@@ -85,4 +85,10 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
       : "memory");
 }
 
+// Programmatic dependent launch: lets the next launch of the stream begin
+// once every CTA has got here; waits for the launch before to have ended
+// (both do nothing in a launch without the attribute).
+__device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace eb

@@ -1233,6 +1233,7 @@ void drop_graphs(eb_sim* s) {
 
 cudaError_t launch_streaming(eb_sim* s, eb::StepArgs& a, bool rec) {
   a.diag = rec ? s->d_diag : nullptr;
+  a.backward = a.in == s->d_state[1] ? 1u : 0u;  // the buffers alternate, and the directions with them
   const int window = s->cfg.step_window;  // 0: the persistent kernel
   if (s->cfg.flags & EB_FLAG_REFERENCE_ROUNDING)
     return eb::launch_rod_step_fp64_reference(a, rec, s->any_damped, window, s->stream);

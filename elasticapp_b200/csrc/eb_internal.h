@@ -158,6 +158,10 @@ struct StepArgs {
   // bound on the polls of a bounded wait for bulk copies (0: the built-in
   // bound); a small value exercises the timeout path
   uint32_t max_polls;
+  // streaming kernel: walk the windows from the last slot to the first.
+  // Alternate launches do, so that a launch starts with the slots the one
+  // before it left in L2
+  uint32_t backward;
 };
 
 // Rods longer than one CTA's capacity run on a pair of CTAs (a thread-block

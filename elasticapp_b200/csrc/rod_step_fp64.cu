@@ -24,12 +24,22 @@
 // neighbouring slot holds no element / Voronoi point and contributes the zero
 // that the reference's ghost slots contribute.
 //
-// Staging: one thread issues a bulk asynchronous copy (TMA, cp.async.bulk)
-// per input field of the window into shared memory, in two stages on two
-// mbarriers: the state and the node mass (all the first drift reads), then
-// the other parameters, which land while the drift's rotation updates run.
-// (Splitting the copies this way took the kernel from 9.97 to 10.9 G
-// element-steps/s; a finer split, one stage per phase, lost a third.)  Both
+// Staging: a warp issues the bulk asynchronous copies (TMA, cp.async.bulk) of
+// the window's input fields into shared memory, a lane a field, in two stages
+// on two mbarriers: the state and the node mass (all the first drift reads),
+// then the other parameters, which land while the drift's rotation updates
+// run.  They are issued before any other load: one thread issuing the 39
+// copies in turn, behind the loads of the slot's metadata and rod, kept the
+// memory system waiting (0.381 ms a step on the 16,384-rod uneven batch, 5.0
+// of 6.5 TB/s; 0.360 with a lane a field, 0.325 with the copies first, 5.9
+// TB/s of algorithmic bytes and 6.3 of traffic).  A fully copied stage per
+// phase, the other way, lost a third.  Alternate launches walk the windows in
+// opposite directions and so begin with slots still in L2 (1.1 M slots: 105.4
+// -> 100.6 us a step before the above), and a launch's first CTAs stage their
+// parameters while the launch before ends (88.2 -> 85.1 us; the wait for it
+// comes before the state is touched).  (Prefetching the next windows into L2
+// meanwhile: 0.396 ms, twice the copies to issue.  The state read as first to
+// be evicted: no change.)  Both
 // waits are bounded; the threads vote on them, and a CTA whose copies did
 // not land in time records it in the status word, waits for the copies it
 // issued and leaves.  The 128-slot windows run 5 CTAs per SM (96 registers a
@@ -51,7 +61,7 @@
 
 #include "bulk_copy.cuh"
 #include "eb_internal.h"
-#include "rod_math.cuh"
+#include "rod_fast.cuh"
 
 namespace eb {
 namespace {
@@ -108,15 +118,15 @@ __device__ __forceinline__ void st3(double* __restrict__ p, int64_t S, int64_t g
 
 __device__ __forceinline__ void so3(double q[9], double u0, double u1, double u2) {
 #ifdef EB_FAST_FP64
-  so3_update_fast(q, u0, u1, u2);
+  rotate(q, rotation(u0, u1, u2));
 #else
   so3_update(q, u0, u1, u2);
 #endif
 }
 
-__device__ __forceinline__ D3 curvature(const double qc[9], const double qn[9], double span) {
+__device__ __forceinline__ D3 voronoi_curvature(const double qc[9], const double qn[9], double span) {
 #ifdef EB_FAST_FP64
-  return inv_rotate_divide_fast(qc, qn, span);
+  return curvature(qc, qn, span);
 #else
   return inv_rotate_divide(qc, qn, span);
 #endif
@@ -135,9 +145,10 @@ __device__ __forceinline__ void clamp_value(const RodInfo& ri, uint32_t hits, ui
   }
 }
 
-template <int W, bool kDiag, bool kDamped, bool kContact>
+template <int W, int MinBlocks, bool kDiag, bool kDamped, bool kContact>
 __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem) {
   using M = RowMap<kDamped, kDiag>;
+  static_assert(kParamFields <= 32 && kStateFields <= 32, "one lane of a warp issues each field's copy");
   constexpr int kTile = W - 4;  // interior slots stored per CTA (even)
   constexpr int kLeftHalo = 2;  // window starts 2 slots left of the tile
   constexpr int kRows = M::rows();
@@ -157,11 +168,41 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + kRows * W);
 
   const int s = threadIdx.x;
-  const int64_t g0 = static_cast<int64_t>(blockIdx.x) * kTile - kLeftHalo;
+  const unsigned tile = a.backward ? gridDim.x - 1u - blockIdx.x : blockIdx.x;
+  const int64_t g0 = static_cast<int64_t>(tile) * kTile - kLeftHalo;
   const int64_t g = g0 + s;
   const int64_t S = a.stride;
   const bool valid = g >= 0 && g < a.n_slots;
   const bool interior = valid && s >= kLeftHalo && s < kLeftHalo + kTile;
+  // ---- stage the window's inputs with bulk copies, one lane a field
+  if (s == 0) {
+    mbar_init(bar, 1);
+    mbar_init(bar + 1, 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  const int64_t lo = g0 < 0 ? 0 : g0;
+  const int64_t hi = (g0 + W < S) ? g0 + W : S;
+  const uint32_t bytes = static_cast<uint32_t>((hi - lo) * sizeof(double));
+  const int off = static_cast<int>(lo - g0);
+  // the state and the node mass (the first drift's inputs) on bar[0], the
+  // other parameters on bar[1], so the drift starts before they land
+  if (s == 0) {
+    mbar_arrive_expect_tx(bar, bytes * static_cast<uint32_t>(kStateFields + 1));
+    mbar_arrive_expect_tx(bar + 1, bytes * static_cast<uint32_t>(kRows - kStateFields - 1));
+  }
+  if (s < 32) __syncwarp();
+  auto copy_parameters = [&]() {
+    if (s < kParamFields && M::needed(s))
+      bulk_g2s(R.row(M::param(s)) + off, a.par + s * S + lo, bytes, s == kMass ? bar : bar + 1);
+  };
+  // (the CTAs that may have to wait; the others need the state first)
+  const bool early = blockIdx.x < 148u * MinBlocks;
+  if (early) copy_parameters();
+  grid_dependency_launch();
+  grid_dependency_wait();
+  if (s < kStateFields) bulk_g2s(R.row(s) + off, a.in + s * S + lo, bytes, bar);
+  if (!early) copy_parameters();
   const uint32_t meta = valid ? a.meta[g] : 0u;
   // per-rod constraint data, fetched while the bulk copies are in flight:
   // the slot's hits (which clamp holds it, the torque, the damper) and the
@@ -175,30 +216,6 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
     damper_r = ri.damper_r;
   }
 
-  // ---- stage the window's inputs with bulk copies (issuing them before the
-  // loads above, which wait on the metadata word, measured no faster)
-  if (s == 0) {
-    mbar_init(bar, 1);
-    mbar_init(bar + 1, 1);
-    mbar_fence_init();
-  }
-  __syncthreads();
-  if (s == 0) {
-    const int64_t lo = g0 < 0 ? 0 : g0;
-    const int64_t hi = (g0 + W < S) ? g0 + W : S;
-    const uint32_t bytes = static_cast<uint32_t>((hi - lo) * sizeof(double));
-    const int off = static_cast<int>(lo - g0);
-    // the state and the node mass (the first drift's inputs) on bar[0], the
-    // other parameters on bar[1], so the drift starts before they land
-    mbar_arrive_expect_tx(bar, bytes * static_cast<uint32_t>(kStateFields + 1));
-#pragma unroll 1
-    for (int f = 0; f < kStateFields; ++f) bulk_g2s(R.row(f) + off, a.in + f * S + lo, bytes, bar);
-    bulk_g2s(R.row(M::param(kMass)) + off, a.par + kMass * S + lo, bytes, bar);
-    mbar_arrive_expect_tx(bar + 1, bytes * static_cast<uint32_t>(kRows - kStateFields - 1));
-#pragma unroll 1
-    for (int f = 0; f < kParamFields; ++f)
-      if (M::needed(f) && f != kMass) bulk_g2s(R.row(M::param(f)) + off, a.par + f * S + lo, bytes, bar + 1);
-  }
   const bool ok0 = wait_copies(a, bar);
 
   const double hdt = a.drift_pre;
@@ -249,15 +266,19 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
     D3 f{0.0, 0.0, 0.0};
     if (elem) {
       const D3 dx = R.get3(rX, s + 1) - x;
-      l = sqrt(dx.x * dx.x + dx.y * dx.y + dx.z * dx.z);
       l0 = R.at(rL0, s);
-      e = l / l0;
 #ifdef EB_FAST_FP64
-      // one reciprocal each of l and e; the dilatation rate (t . dv) / (e l0)
-      // as (t . dv) / l (e l0 = l)
-      const double il = 1.0 / l, ie = 1.0 / e;
+      // one reciprocal each of l and e (rod_fast.cuh); the dilatation rate
+      // (t . dv) / (e l0) as (t . dv) / l (e l0 = l)
+      const Length len = length_of(dx.x * dx.x + dx.y * dx.y + dx.z * dx.z);
+      l = len.l;
+      const double il = len.il;
+      e = div_from(l, l0, rcp_from(l0, rcp_near(l0)));
+      const double ie = rcp_from(e, l0 * il);
       t = scale(dx, il);
 #else
+      l = sqrt(dx.x * dx.x + dx.y * dx.y + dx.z * dx.z);
+      e = l / l0;
       t = divide(dx, l);
 #endif
       const D3 qt = matvec(q, t);
@@ -301,13 +322,14 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
 #pragma unroll
       for (int k = 0; k < 9; ++k) qn[k] = R.at(rQ + k, s + 1);
       const double D0 = R.at(rD0, s);
-      kappa = curvature(q, qn, D0);
+      kappa = voronoi_curvature(q, qn, D0);
       const double D = 0.5 * (l + R.at(rL, s + 1));
-      eps = D / D0;
 #ifdef EB_FAST_FP64
-      const double ie = D0 / D;  // 1 / eps
+      if (kDiag) eps = D / D0;
+      const double ie = div_from(D0, D, rcp_from(D, rcp_near(D)));  // 1 / eps
       const double ic = ie * ie * ie;
 #else
+      eps = D / D0;
       const double ic = 1.0 / (eps * eps * eps);
 #endif
       const D3 dk = kappa - R.get3(rKap0, s);
@@ -350,7 +372,11 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
     const double* __restrict__ jf = a.joint_force;
     Fe = {Fe.x + jf[g], Fe.y + jf[S + g], Fe.z + jf[2 * S + g]};
   }
+#ifdef EB_FAST_FP64
+  const double inv_m = rcp_from(m, rcp_near(m));
+#else
   const double inv_m = 1.0 / m;
+#endif
   const D3 acc = {(F.x + Fe.x) * inv_m, (F.y + Fe.y) * inv_m, (F.z + Fe.z) * inv_m};
 
   D3 T{0.0, 0.0, 0.0}, alpha{0.0, 0.0, 0.0};
@@ -413,7 +439,9 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
       if (meta & kLastElem) em += 0.5 * mn;
       const double nur = damper_r;
 #ifdef EB_FAST_FP64
-      w = {w.x * exp(e * (-nur * em * jinv.x * ddt)), w.y * exp(e * (-nur * em * jinv.y * ddt)),
+      // (a circular cross section: one factor for both bending directions)
+      const double ex = exp(e * (-nur * em * jinv.x * ddt));
+      w = {w.x * ex, w.y * (jinv.y == jinv.x ? ex : exp(e * (-nur * em * jinv.y * ddt))),
            w.z * exp(e * (-nur * em * jinv.z * ddt))};
 #else
       w = {w.x * pow(exp(-nur * em * jinv.x * ddt), e), w.y * pow(exp(-nur * em * jinv.y * ddt), e),
@@ -460,7 +488,7 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
 template <int W, int MinBlocks, bool kDiag, bool kDamped, bool kContact>
 __global__ void __launch_bounds__(W, MinBlocks) rod_step_fp64_kernel(const StepArgs a) {
   extern __shared__ __align__(128) double smem[];
-  rod_step_window<W, kDiag, kDamped, kContact>(a, smem);
+  rod_step_window<W, MinBlocks, kDiag, kDamped, kContact>(a, smem);
 }
 
 template <int W, int MinBlocks, bool kDiag, bool kDamped, bool kContact>
@@ -473,8 +501,19 @@ cudaError_t launch_variant(const StepArgs& args, cudaStream_t stream) {
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
   if (e != cudaSuccess) return e;
   const unsigned grid = static_cast<unsigned>((args.n_slots + kTile - 1) / kTile);
-  kern<<<grid, W, bytes, stream>>>(args);
-  return cudaGetLastError();
+  // programmatic launch: the windows' parameters may be staged while the
+  // launch before ends (the kernel waits for it before it touches the state)
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(grid);
+  lc.blockDim = dim3(W);
+  lc.dynamicSmemBytes = bytes;
+  lc.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  lc.attrs = at;
+  lc.numAttrs = 1;
+  return cudaLaunchKernelEx(&lc, kern, args);
 }
 
 template <int W, int MinBlocks, bool kContact>
