@@ -163,6 +163,7 @@ struct JointDevice {
   int32_t *force_src = nullptr, *torque_src = nullptr;
   int64_t n_force = 0, n_torque = 0;
   double* loads = nullptr;  // 6 x stride: node force rows 0-2, element torque rows 3-5 (lab frame)
+  int32_t max_per_slot = 0;
 };
 
 }  // namespace
@@ -1049,6 +1050,8 @@ eb_status setup_joints(eb_sim* s) {
   EB_CUDA(cudaMalloc(reinterpret_cast<void**>(&j.out), dev.size() * 6 * sizeof(double)));
   EB_CUDA(cudaMalloc(reinterpret_cast<void**>(&j.loads), static_cast<size_t>(6 * S) * sizeof(double)));
   EB_CUDA(cudaMemsetAsync(j.loads, 0, static_cast<size_t>(6 * S) * sizeof(double), s->stream));
+  for (const auto* m : {&fsrc, &tsrc})
+    for (const auto& kv : *m) j.max_per_slot = std::max(j.max_per_slot, static_cast<int32_t>(kv.second.size()));
   j.n_force = static_cast<int64_t>(fslot.size());
   j.n_torque = static_cast<int64_t>(tslot.size());
   j.on = true;
@@ -1059,6 +1062,7 @@ eb::JointArgs joint_args(eb_sim* s) {
   const JointDevice& j = s->jd;
   eb::JointArgs a{};
   a.n_joints = static_cast<int32_t>(s->joints.size());
+  a.max_per_slot = j.max_per_slot;
   a.joints = j.joints;
   a.out = j.out;
   a.stride = s->stride;
@@ -1801,8 +1805,7 @@ eb_status step_with_contact(eb_sim* s, double dt, int64_t n_steps, bool diag) {
         if (s->jd.on) {
           ja.state = s->d_state[s->cur];
           ja.pre = a.drift_pre;
-          EB_CUDA(eb::launch_joints(ja, s->stream));
-          s->launches += 2;
+          EB_CUDA(eb::launch_joints(ja, s->stream, &s->launches));
         }
         a.in = s->d_state[s->cur];
         a.out = s->d_state[s->cur ^ 1];

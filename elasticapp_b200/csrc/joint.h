@@ -22,6 +22,7 @@ struct JointDev {
 
 struct JointArgs {
   int32_t n_joints;
+  int32_t max_per_slot;  // most joints acting on one slot
   const JointDev* joints;
   double* out;  // 6 per joint: force (3), lab-frame torque (3)
   const double* state;
@@ -42,6 +43,7 @@ struct JointArgs {
   double* joint_torque;  // 3 x stride, element slots
 };
 
-cudaError_t launch_joints(const JointArgs& a, cudaStream_t stream);
+// launches counted into *launches
+cudaError_t launch_joints(const JointArgs& a, cudaStream_t stream, int64_t* launches);
 
 }  // namespace eb
