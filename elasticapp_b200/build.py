@@ -34,9 +34,11 @@ SOURCES = [
     # joint loads rounded as written, like the CPU restatement
     ("connection.o", "connection.cu", ["--fmad=false"]),
     ("serve.o", "serve.cu", []),
+    # rounded as written, like the host's initial data
+    ("rod_init.o", "rod_init.cu", ["--fmad=false"]),
     ("partition.o", "partition.cu", []),
 ]
-HEADERS = ["eb_internal.h", "rod_math.cuh", "rod_fast.cuh", "bulk_copy.cuh", "contact.h", "eb_host.h", "joint.h"]
+HEADERS = ["eb_internal.h", "rod_math.cuh", "rod_fast.cuh", "bulk_copy.cuh", "contact.h", "eb_host.h", "joint.h", "rod_init.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

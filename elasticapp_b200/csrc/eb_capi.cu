@@ -279,7 +279,10 @@ void cross3(const double m[3], const double v[3], double o[3]) {
 // CircleCrossSectionOperations.hpp:84-132), rigidities
 // (LinearHyperElasticityFacade.hpp:273-327; Initializers/detail/Elasticity.hpp:
 // 54-77) and kinematics (WithRodKinematics.hpp:344-424).
-eb_status init_straight_rod(const eb_straight_rod& p, RodHost& r) {
+//
+// The checks of its arguments, the unit tangent, the node spacing (per
+// component) and the directors' rows:
+eb_status straight_rod_frame(const eb_straight_rod& p, double t[3], double step[3], double rows[9]) {
   const int64_t n = p.n_elements;
   if (n < 2) return fail(EB_ERR_INVALID_ARGUMENT, "a rod needs at least 2 elements");
   if (!(p.radius > 0.0) || !(p.length > 0.0) || !(p.density > 0.0))
@@ -291,11 +294,33 @@ eb_status init_straight_rod(const eb_straight_rod& p, RodHost& r) {
   const double dn = norm3(p.direction), nn = norm3(p.normal);
   if (dn == 0.0) return fail(EB_ERR_INVALID_ARGUMENT, "direction is zero");
   if (nn == 0.0) return fail(EB_ERR_INVALID_ARGUMENT, "normal is zero");
-  const double t[3] = {p.direction[0] / dn, p.direction[1] / dn, p.direction[2] / dn};
+  for (int d = 0; d < 3; ++d) t[d] = p.direction[d] / dn;
   const double nv[3] = {p.normal[0] / nn, p.normal[1] / nn, p.normal[2] / nn};
   if (std::fabs(t[0] * nv[0] + t[1] * nv[1] + t[2] * nv[2]) > 1e-10)
     return fail(EB_ERR_INVALID_ARGUMENT, "the proposed normal and tangent are non-orthogonal");
 
+  for (int d = 0; d < 3; ++d) {
+    const double stop = p.origin[d] + p.length * t[d];
+    step[d] = (stop - p.origin[d]) / static_cast<double>(n);
+  }
+  double v1[3] = {nv[0], nv[1], nv[2]}, v2[3], v3[3], tmp[3];
+  cross3(t, nv, v2);
+  cross3(v1, v2, v3);
+  cross3(v3, v1, tmp);
+  std::memcpy(v2, tmp, sizeof(tmp));
+  const double n2 = norm3(v2), n3 = norm3(v3);
+  for (int d = 0; d < 3; ++d) {
+    rows[d] = v1[d];
+    rows[3 + d] = v2[d] / n2;
+    rows[6 + d] = v3[d] / n3;
+  }
+  return EB_OK;
+}
+
+eb_status init_straight_rod(const eb_straight_rod& p, RodHost& r) {
+  double t[3], step[3], rows[9];
+  if (eb_status st = straight_rod_frame(p, t, step, rows)) return st;
+  const int64_t n = p.n_elements;
   r.n = n;
   r.model = p.model;
   const int64_t W = n + 1;
@@ -305,19 +330,8 @@ eb_status init_straight_rod(const eb_straight_rod& p, RodHost& r) {
   auto S = [&](int f, int64_t j) -> double& { return r.state[static_cast<size_t>(f * W + j)]; };
   auto P = [&](int f, int64_t j) -> double& { return r.param[static_cast<size_t>(f * W + j)]; };
 
-  for (int d = 0; d < 3; ++d) {
-    const double stop = p.origin[d] + p.length * t[d];
-    const double step = (stop - p.origin[d]) / static_cast<double>(n);
-    for (int64_t j = 0; j <= n; ++j) S(eb::kStX + d, j) = p.origin[d] + static_cast<double>(j) * step;
-  }
-  double v1[3] = {nv[0], nv[1], nv[2]}, v2[3], v3[3], tmp[3];
-  cross3(t, nv, v2);
-  cross3(v1, v2, v3);
-  cross3(v3, v1, tmp);
-  std::memcpy(v2, tmp, sizeof(tmp));
-  const double n2 = norm3(v2), n3 = norm3(v3);
-  const double rows[9] = {v1[0],      v1[1],      v1[2],      v2[0] / n2, v2[1] / n2,
-                          v2[2] / n2, v3[0] / n3, v3[1] / n3, v3[2] / n3};
+  for (int d = 0; d < 3; ++d)
+    for (int64_t j = 0; j <= n; ++j) S(eb::kStX + d, j) = p.origin[d] + static_cast<double>(j) * step[d];
   for (int k = 0; k < 9; ++k)
     for (int64_t i = 0; i < n; ++i) S(eb::kStQ + k, i) = rows[k];
 
@@ -613,13 +627,18 @@ eb_status setup_contact(eb_sim* s) {
 namespace eb {
 void set_last_error(const std::string& message) { g_last_error = message; }
 
-eb_status host_straight_rod(const eb_straight_rod& p, HostRodData& out) {
-  RodHost r;
-  if (eb_status st = init_straight_rod(p, r)) return st;
-  out.n = r.n;
-  out.damped = r.model == EB_ROD_DAMPED;
-  out.state = std::move(r.state);
-  out.param = std::move(r.param);
+eb_status straight_rod_spec(const eb_straight_rod& p, RodSpec& out) {
+  double t[3];
+  if (eb_status st = straight_rod_frame(p, t, out.step, out.rows)) return st;
+  for (int d = 0; d < 3; ++d) out.origin[d] = p.origin[d];
+  out.area = static_cast<double>(M_PI) * (p.radius * p.radius);
+  out.density = p.density;
+  out.youngs = p.youngs_modulus;
+  out.shear = p.shear_modulus;
+  out.damped = p.model == EB_ROD_DAMPED ? 1 : 0;
+  out.nu_f = out.damped ? p.force_damping_rate : 0.0;
+  out.nu_t = out.damped ? p.torque_damping_rate : 0.0;
+  out.n = static_cast<int32_t>(p.n_elements);
   return EB_OK;
 }
 }  // namespace eb

@@ -4,22 +4,16 @@
 
 #include <cstdint>
 #include <string>
-#include <vector>
 
 #include "../../include/elastica_b200.h"
 #include "eb_internal.h"
+#include "rod_init.h"
 
 namespace eb {
 
-// One straight rod from its initializer, in the local slot layout: field row f
-// of the rod at [f * (n + 1), (f + 1) * (n + 1)).
-struct HostRodData {
-  int64_t n = 0;
-  bool damped = false;
-  std::vector<double> state;  // kStateFields rows
-  std::vector<double> param;  // kParamFields rows
-};
-eb_status host_straight_rod(const eb_straight_rod& p, HostRodData& out);
+// A straight rod's initializer (the checks of its arguments, and the part of
+// its initial data that is computed once a rod; rod_init.cu has the rest)
+eb_status straight_rod_spec(const eb_straight_rod& p, RodSpec& out);
 
 // records the message eb_last_error() returns on this thread
 void set_last_error(const std::string& message);

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "eb_internal.h"
+#include "rod_init.h"
 #include "rod_math.cuh"
 
 namespace eb {
@@ -86,37 +87,37 @@ __global__ void rod_energy_kernel(int64_t n_rods, int64_t S, const int64_t* __re
   }
 }
 
-// rods given by their first slot and element count; out[5 r + 4] is the
-// gravitational potential -sum m g.x of rod r
-__global__ void rod_energy_list_kernel(int64_t n_rods, int64_t S, const int64_t* __restrict__ start,
-                                       const int32_t* __restrict__ n_el, const double* __restrict__ st,
-                                       const double* __restrict__ par, double g0, double g1, double g2,
+// listed rods, given by their first slot and element count; out[5 r + 4] is
+// the gravitational potential -sum m g.x of rod r
+__global__ void rod_energy_list_kernel(const RodRef* __restrict__ refs, int64_t count, int64_t S,
+                                       const int64_t* __restrict__ start, const int32_t* __restrict__ n_el,
+                                       const double* __restrict__ st, const double* __restrict__ par,
                                        double* __restrict__ out) {
   const int64_t warp = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= n_rods) return;
-  const double gvec[3] = {g0, g1, g2};
+  if (warp >= count) return;
+  const int64_t rod = refs[warp].rod;
+  const double gvec[3] = {refs[warp].gravity[0], refs[warp].gravity[1], refs[warp].gravity[2]};
   double et, er, es, eb, ep;
-  rod_energy_warp(start[warp], n_el[warp], S, st, par, gvec, et, er, es, eb, ep);
+  rod_energy_warp(start[rod], n_el[rod], S, st, par, gvec, et, er, es, eb, ep);
   if (lane == 0) {
-    out[5 * warp + 0] = 0.5 * et;
-    out[5 * warp + 1] = 0.5 * er;
-    out[5 * warp + 2] = 0.5 * es;
-    out[5 * warp + 3] = 0.5 * eb;
-    out[5 * warp + 4] = ep;
+    out[5 * rod + 0] = 0.5 * et;
+    out[5 * rod + 1] = 0.5 * er;
+    out[5 * rod + 2] = 0.5 * es;
+    out[5 * rod + 3] = 0.5 * eb;
+    out[5 * rod + 4] = ep;
   }
 }
 
 }  // namespace
 
-cudaError_t launch_rod_energy_list(int64_t n_rods, int64_t stride, const int64_t* start, const int32_t* n_el,
-                                   const double* state, const double* params, const double gravity[3], double* out,
+cudaError_t launch_rod_energy_list(const RodRef* refs, int64_t count, int64_t stride, const int64_t* rod_start,
+                                   const int32_t* rod_n, const double* state, const double* params, double* out,
                                    cudaStream_t stream) {
-  if (n_rods <= 0) return cudaSuccess;
-  constexpr int kThreads = 256;
-  const unsigned grid = static_cast<unsigned>((n_rods * 32 + kThreads - 1) / kThreads);
-  rod_energy_list_kernel<<<grid, kThreads, 0, stream>>>(n_rods, stride, start, n_el, state, params, gravity[0],
-                                                        gravity[1], gravity[2], out);
+  if (count <= 0) return cudaSuccess;
+  constexpr int kThreads = 64;  // two rods a CTA: a warp's rod is a chain of latencies, so spread them
+  const unsigned grid = static_cast<unsigned>((count * 32 + kThreads - 1) / kThreads);
+  rod_energy_list_kernel<<<grid, kThreads, 0, stream>>>(refs, count, stride, rod_start, rod_n, state, params, out);
   return cudaGetLastError();
 }
 

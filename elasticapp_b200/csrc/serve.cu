@@ -6,8 +6,8 @@
 // HBM budget at creation.  A request is admitted when enough bins are free:
 // its rods are packed into its own bins (next fit; a rod of 520 to 1039
 // elements takes a pair of adjacent bins, run by a cluster of two CTAs),
-// initialised on the host and copied in, and its initial energy is computed
-// on the device.  Every tick is one launch of the resident kernel per
+// initialised on the device (rod_init.cu), and its initial energy is computed
+// there.  Every tick is one launch of the resident kernel per
 // precision (mixed, and FP64 for requests that fell back) over the bins of
 // every active request: each CTA reads its bin, step count, time step and
 // environment from a per-CTA table, so requests of different sizes, time
@@ -41,15 +41,13 @@
 #include "../../include/elastica_b200.h"
 #include "eb_host.h"
 #include "eb_internal.h"
+#include "rod_init.h"
 
 namespace eb {
 cudaError_t launch_rod_block_mixed_serve(const StepArgs& args, const ServeCta* serve, int n_ctas, int n_steps,
                                          bool damped, cudaStream_t stream);
 cudaError_t launch_rod_block_fp64_serve(const StepArgs& args, const ServeCta* serve, int n_ctas, int n_steps,
                                         bool damped, cudaStream_t stream);
-cudaError_t launch_rod_energy_list(int64_t n_rods, int64_t stride, const int64_t* start, const int32_t* n_el,
-                                   const double* state, const double* params, const double gravity[3], double* out,
-                                   cudaStream_t stream);
 }  // namespace eb
 
 namespace {
@@ -64,7 +62,7 @@ constexpr int64_t kBinFill = 512;
 constexpr int64_t kPairFill = 2 * kBinFill;
 constexpr int64_t kRodsPerBin = kBin / 3;     // a rod takes at least 3 slots
 constexpr size_t kArenaBytes = size_t(1) << 30;  // pinned result arena
-constexpr size_t kUploadBytes = size_t(1) << 28;  // pinned staging of admitted requests' initial data
+constexpr size_t kUploadBytes = size_t(1) << 27;  // pinned staging of admitted requests' initial data
 using Clock = std::chrono::steady_clock;
 
 eb_status fail(eb_status st, const std::string& m) {
@@ -248,6 +246,7 @@ struct eb_server {
   // pinned staging of initial data: copies from pageable memory would wait
   // for the stream (the running ticks) before each admission
   Ring upload;
+  unsigned char* d_upload = nullptr;  // the device's copy of it
   std::deque<cudaEvent_t> upload_events;  // one per live upload allocation, in order
   std::vector<cudaEvent_t> spare_events;
   BinPool bins;
@@ -267,7 +266,7 @@ namespace {
 void server_free(eb_server* s) {
   cudaSetDevice(s->cfg.device);
   if (s->stream) cudaStreamSynchronize(s->stream);
-  void* dev[] = {s->state[0], s->state[1], s->par, s->meta, s->rods, s->rod_start, s->rod_n, s->e0, s->e1, s->status};
+  void* dev[] = {s->state[0], s->state[1], s->par, s->meta, s->rods, s->rod_start, s->rod_n, s->e0, s->e1, s->status, s->d_upload};
   for (void* p : dev)
     if (p) cudaFree(p);
   for (int a = 0; a < 2; ++a)
@@ -366,128 +365,104 @@ eb_status upload_alloc(eb_server* s, size_t bytes, size_t* off) {
   return EB_OK;
 }
 
-// Copy the request's initial rods into its bins (through pinned staging, so
-// the copies queue behind the running ticks instead of waiting for them) and
-// compute its initial energy.
-eb_status place(eb_server* s, Request& r) {
-  const int64_t S = s->stride;
-  const size_t nu = r.bin_count.size(), nr = r.rods.size();
-  auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-  std::vector<size_t> ust(nu), upr(nu), umt(nu);
-  size_t bytes = 0;
-  for (size_t b = 0; b < nu; ++b) {
-    const size_t c = static_cast<size_t>(r.bin_count[b]);
-    ust[b] = bytes;
-    bytes += up(c * eb::kStateFields * sizeof(double));
-    upr[b] = bytes;
-    bytes += up(c * eb::kParamFields * sizeof(double));
-    umt[b] = bytes;
-    bytes += up(c * sizeof(uint32_t));
+// Staging space for `bytes`, copied (by stage_copy) to the same place of the
+// device's copy of the ring; close_stage records when it may be reused (on
+// every path, so the ring's allocations and the events stay paired).
+eb_status close_stage(eb_server* s) {
+  cudaEvent_t ev = nullptr;
+  if (!s->spare_events.empty()) {
+    ev = s->spare_events.back();
+    s->spare_events.pop_back();
+  } else {
+    SV_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   }
-  const size_t uinfo = bytes;
-  bytes += up(nr * sizeof(eb::RodInfo));
-  const size_t ustart = bytes;
-  bytes += up(nr * sizeof(int64_t));
-  const size_t un = bytes;
-  bytes += up(nr * sizeof(int32_t));
-  size_t base_off = 0;
-  if (eb_status st = upload_alloc(s, bytes, &base_off)) return st;
-  unsigned char* base = s->upload.base + base_off;
-  std::vector<double*> st(nu), pr(nu);
-  std::vector<uint32_t*> mt(nu);
-  for (size_t b = 0; b < nu; ++b) {
-    st[b] = reinterpret_cast<double*>(base + ust[b]);
-    pr[b] = reinterpret_cast<double*>(base + upr[b]);
-    mt[b] = reinterpret_cast<uint32_t*>(base + umt[b]);
-  }
-  eb::RodInfo* info = reinterpret_cast<eb::RodInfo*>(base + uinfo);
-  int64_t* rstart = reinterpret_cast<int64_t*>(base + ustart);
-  int32_t* rn = reinterpret_cast<int32_t*>(base + un);
-  // the staging space is reused once this event has passed (recorded on
-  // every path, so the ring's allocations and the events stay paired)
-  auto close_upload = [&]() -> eb_status {
-    cudaEvent_t ev = nullptr;
-    if (!s->spare_events.empty()) {
-      ev = s->spare_events.back();
-      s->spare_events.pop_back();
-    } else {
-      SV_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-    }
-    s->upload_events.push_back(ev);
-    SV_CUDA(cudaEventRecord(ev, s->stream));
-    return EB_OK;
-  };
-  size_t voff = 0;
-  for (size_t k = 0; k < r.rods.size(); ++k) {
-    eb::HostRodData h;
-    if (eb_status e = eb::host_straight_rod(r.rods[k], h)) {
-      close_upload();
-      return e;
-    }
-    const int64_t n = h.n, W = n + 1, b = r.rod_bin[k], o = r.rod_off[k], c = r.bin_count[b];
-    if (!r.velocities.empty()) {
-      for (int d = 0; d < 3; ++d)
-        for (int64_t j = 0; j <= n; ++j) h.state[(eb::kStV + d) * W + j] = r.velocities[voff + d * W + j];
-      voff += static_cast<size_t>(3 * W);
-    }
-    // (a unit's rods fill its slots [0, c) without gaps: every staged entry is written)
-    for (int f = 0; f < eb::kStateFields; ++f)
-      std::memcpy(&st[b][f * c + o], &h.state[f * W], W * sizeof(double));
-    for (int f = 0; f < eb::kParamFields; ++f)
-      std::memcpy(&pr[b][f * c + o], &h.param[f * W], W * sizeof(double));
-    const int64_t rid = r.rod0 + static_cast<int64_t>(k);
-    for (int64_t j = 0; j <= n; ++j) {
-      uint32_t m = static_cast<uint32_t>(rid) << eb::kRodShift;
-      if (j < n) m |= eb::kElem;
-      if (j < n - 1) m |= eb::kVor;
-      if (j == 0) m |= eb::kFirst;
-      if (j == n) m |= eb::kLastNode;
-      if (j == n - 1) m |= eb::kLastElem;
-      mt[b][o + j] = m;
-    }
-    eb::RodInfo& ri = info[k];
-    std::memset(&ri, 0, sizeof(ri));
-    for (int d = 0; d < 3; ++d) ri.clamp_x[d] = h.state[(eb::kStX + d) * W];
-    for (int q = 0; q < 9; ++q) ri.clamp_Q[q] = h.state[(eb::kStQ + q) * W];
-    ri.damper_t = 1.0;
-    ri.clamp_slot[1] = -1;
-    ri.torque_slot = -1;
-    ri.clamp_slot[0] = -1;
-    if (r.options & EB_REQUEST_CLAMP) {
-      ri.flags |= eb::kRodClamp;
-      ri.clamp_slot[0] = r.bins[b] * kBin + o;  // node 0 / element 0 of the rod
-    }
-    if (r.options & EB_REQUEST_DAMPER) {
-      ri.flags |= eb::kRodDamper;
-      ri.damper_t = std::exp(-r.nu_t * r.dt);
-      ri.damper_r = r.nu_r;
-    }
-    rstart[k] = r.bins[b] * kBin + o;
-    rn[k] = static_cast<int32_t>(n);
-    if (h.damped) r.damped = true;
-  }
-  for (size_t b = 0; b < r.bin_count.size(); ++b) {
-    const int64_t c = r.bin_count[b], g0 = r.bins[b] * kBin;
-    const size_t pitch = static_cast<size_t>(S) * sizeof(double), w = static_cast<size_t>(c) * sizeof(double);
-    SV_CUDA(cudaMemcpy2DAsync(s->state[s->cur] + g0, pitch, st[b], w, w, eb::kStateFields,
-                              cudaMemcpyHostToDevice, s->stream));
-    SV_CUDA(cudaMemcpy2DAsync(s->par + g0, pitch, pr[b], w, w, eb::kParamFields, cudaMemcpyHostToDevice,
-                              s->stream));
-    SV_CUDA(cudaMemcpyAsync(s->meta + g0, mt[b], c * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream));
-  }
-  SV_CUDA(cudaMemcpyAsync(s->rods + r.rod0, info, nr * sizeof(eb::RodInfo), cudaMemcpyHostToDevice, s->stream));
-  SV_CUDA(cudaMemcpyAsync(s->rod_start + r.rod0, rstart, nr * sizeof(int64_t), cudaMemcpyHostToDevice, s->stream));
-  SV_CUDA(cudaMemcpyAsync(s->rod_n + r.rod0, rn, nr * sizeof(int32_t), cudaMemcpyHostToDevice, s->stream));
-  if (eb_status st = close_upload()) return st;
-  const double g[3] = {(r.options & EB_REQUEST_GRAVITY) ? r.gravity[0] : 0.0,
-                       (r.options & EB_REQUEST_GRAVITY) ? r.gravity[1] : 0.0,
-                       (r.options & EB_REQUEST_GRAVITY) ? r.gravity[2] : 0.0};
-  SV_CUDA(eb::launch_rod_energy_list(static_cast<int64_t>(nr), S, s->rod_start + r.rod0, s->rod_n + r.rod0,
-                                     s->state[s->cur], s->par, g, s->e0 + 5 * r.rod0, s->stream));
+  s->upload_events.push_back(ev);
+  SV_CUDA(cudaEventRecord(ev, s->stream));
   return EB_OK;
 }
 
+eb::RodRef rod_ref(const Request& r, size_t k) {
+  eb::RodRef ref{};
+  ref.rod = r.rod0 + static_cast<int64_t>(k);
+  if (r.options & EB_REQUEST_GRAVITY)
+    for (int d = 0; d < 3; ++d) ref.gravity[d] = r.gravity[d];
+  return ref;
+}
+
+size_t spec_bytes(size_t rods) { return (rods * (sizeof(eb::RodSpec) + sizeof(eb::RodRef)) + 255) / 256 * 256; }
+
+// Write the initial rods of the requests admitted together into their bins:
+// the rods' specifications and velocities go through pinned staging (so the
+// copy queues behind the running ticks instead of waiting for them), a kernel
+// computes the slots' data there, and another the initial energies.
+eb_status place(eb_server* s, const std::vector<Request*>& batch) {
+  size_t nr = 0, nv = 0;
+  for (const Request* r : batch) {
+    nr += r->rods.size();
+    nv += r->velocities.size();
+  }
+  if (nr == 0) return EB_OK;
+  const size_t uvel = spec_bytes(nr), bytes = uvel + nv * sizeof(double);
+  size_t base_off = 0;
+  if (eb_status st = upload_alloc(s, bytes, &base_off)) return st;
+  unsigned char* base = s->upload.base + base_off;
+  eb::RodSpec* specs = reinterpret_cast<eb::RodSpec*>(base);
+  eb::RodRef* refs = reinterpret_cast<eb::RodRef*>(specs + nr);
+  size_t voff = 0, at = 0;
+  for (Request* r : batch) {
+    const size_t v0 = voff;
+    for (size_t k = 0; k < r->rods.size(); ++k, ++at) {
+      eb::RodSpec spec{};
+      if (eb_status e = eb::straight_rod_spec(r->rods[k], spec)) {
+        close_stage(s);
+        return e;
+      }
+      const int64_t first = r->bins[r->rod_bin[k]] * kBin + r->rod_off[k];
+      spec.start = first;
+      spec.rod = static_cast<uint32_t>(r->rod0 + static_cast<int64_t>(k));
+      spec.velocity = -1;
+      if (!r->velocities.empty()) {
+        spec.velocity = static_cast<int64_t>(voff);
+        voff += static_cast<size_t>(3 * (spec.n + 1));
+      }
+      eb::RodInfo& ri = spec.info;
+      for (int d = 0; d < 3; ++d) ri.clamp_x[d] = spec.origin[d] + 0.0 * spec.step[d];
+      for (int q = 0; q < 9; ++q) ri.clamp_Q[q] = spec.rows[q];
+      ri.damper_t = 1.0;
+      ri.clamp_slot[0] = ri.clamp_slot[1] = -1;
+      ri.torque_slot = -1;
+      if (r->options & EB_REQUEST_CLAMP) {
+        ri.flags |= eb::kRodClamp;
+        ri.clamp_slot[0] = first;  // node 0 / element 0 of the rod
+      }
+      if (r->options & EB_REQUEST_DAMPER) {
+        ri.flags |= eb::kRodDamper;
+        ri.damper_t = std::exp(-r->nu_t * r->dt);
+        ri.damper_r = r->nu_r;
+      }
+      if (spec.damped) r->damped = true;
+      specs[at] = spec;
+      refs[at] = rod_ref(*r, k);
+    }
+    if (voff > v0)
+      std::memcpy(base + uvel + v0 * sizeof(double), r->velocities.data(), (voff - v0) * sizeof(double));
+  }
+  unsigned char* dev = s->d_upload + base_off;
+  SV_CUDA(cudaMemcpyAsync(dev, base, bytes, cudaMemcpyHostToDevice, s->stream));
+  const eb::RodSpec* dspecs = reinterpret_cast<const eb::RodSpec*>(dev);
+  const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(dspecs + nr);
+  SV_CUDA(eb::launch_rod_init(dspecs, static_cast<int64_t>(nr), reinterpret_cast<const double*>(dev + uvel), s->stride,
+                              s->state[s->cur], s->par, s->meta, s->rods, s->rod_start, s->rod_n, s->stream));
+  SV_CUDA(eb::launch_rod_energy_list(drefs, static_cast<int64_t>(nr), s->stride, s->rod_start, s->rod_n,
+                                     s->state[s->cur], s->par, s->e0, s->stream));
+  return close_stage(s);
+}
+
+// Admit what fits, first come first served; the requests admitted in one tick
+// are placed together (as much at a time as half the staging ring holds).
 eb_status admit(eb_server* s) {
+  std::vector<Request*> batch;
+  size_t bytes = 0;
   while (!s->queue.empty()) {
     Request& r = *s->queue.front();
     pack(r);
@@ -504,61 +479,105 @@ eb_status admit(eb_server* s) {
       if (!r.bin_pair[b]) r.bins[b] = s->bins.take_single();
     r.steps_done = 0;
     r.damped = false;
-    if (eb_status e = place(s, r)) return e;
+    const size_t need = spec_bytes(r.rods.size()) + r.velocities.size() * sizeof(double);
+    if (!batch.empty() && bytes + need > kUploadBytes / 2) {
+      if (eb_status e = place(s, batch)) return e;
+      batch.clear();
+      bytes = 0;
+    }
+    batch.push_back(&r);
+    bytes += need;
     if (r.queued_s < 0.0) r.queued_s = std::chrono::duration<double>(Clock::now() - r.t_submit).count();
     r.state = kActive;
     s->queue.pop_front();
     s->active.push_back(&r);
   }
-  return EB_OK;
+  return place(s, batch);
 }
 
 eb_status poll_events(eb_server* s, bool block_oldest);
 
-// Enqueue the retirement of a request whose last step ran in this tick.
-eb_status retire(eb_server* s, Request& r) {
-  const int64_t S = s->stride, nr = static_cast<int64_t>(r.rods.size());
-  const double g[3] = {(r.options & EB_REQUEST_GRAVITY) ? r.gravity[0] : 0.0,
-                       (r.options & EB_REQUEST_GRAVITY) ? r.gravity[1] : 0.0,
-                       (r.options & EB_REQUEST_GRAVITY) ? r.gravity[2] : 0.0};
-  SV_CUDA(eb::launch_rod_energy_list(nr, S, s->rod_start + r.rod0, s->rod_n + r.rod0, s->state[s->cur], s->par, g,
-                                     s->e1 + 5 * r.rod0, s->stream));
-  size_t slots = 0;
-  for (int32_t c : r.bin_count) slots += static_cast<size_t>(c);
-  const size_t bytes = (slots * eb::kStateFields + 10 * static_cast<size_t>(nr)) * sizeof(double);
-  size_t off = 0;
-  while (!s->arena.alloc(bytes, &off)) {
-    if (s->finishing.empty()) return fail(EB_ERR_OUT_OF_MEMORY, "request result larger than the host arena");
-    // the arena is full: wait for the oldest retirement and take it out
-    if (eb_status st = poll_events(s, true)) return st;
+// Enqueue the retirement of requests whose last step ran in this tick, for
+// which the arena has room: their final energies, then their results into the
+// arena, a launch each for all of them.
+eb_status retire_batch(eb_server* s, const std::vector<Request*>& batch) {
+  size_t nr = 0;
+  for (const Request* r : batch) nr += r->rods.size();
+  if (nr == 0) return EB_OK;
+  const size_t bytes = nr * sizeof(eb::RodRef);
+  size_t base_off = 0;
+  if (eb_status st = upload_alloc(s, bytes, &base_off)) return st;
+  eb::RodRef* refs = reinterpret_cast<eb::RodRef*>(s->upload.base + base_off);
+  for (Request* r : batch) {
+    double* dst = reinterpret_cast<double*>(s->arena.base + r->arena_off);
+    int64_t at = 0;
+    r->result_off.assign(r->rods.size(), 0);
+    for (size_t k = 0; k < r->rods.size(); ++k) {
+      r->result_off[k] = at;
+      at += eb::kStateFields * (r->rods[k].n_elements + 1);
+    }
+    for (size_t k = 0; k < r->rods.size(); ++k) {
+      eb::RodRef ref = rod_ref(*r, k);
+      ref.result = dst + r->result_off[k];
+      ref.energies = dst + at + 5 * k;
+      ref.final_at = 5 * static_cast<int64_t>(r->rods.size());
+      *refs++ = ref;
+    }
   }
-  r.arena_off = off;
-  double* dst = reinterpret_cast<double*>(s->arena.base + off);
-  size_t pos = 0;
-  for (size_t b = 0; b < r.bin_count.size(); ++b) {
-    const int64_t c = r.bin_count[b], g0 = r.bins[b] * kBin;
-    const size_t w = static_cast<size_t>(c) * sizeof(double);
-    SV_CUDA(cudaMemcpy2DAsync(dst + pos, w, s->state[s->cur] + g0, static_cast<size_t>(S) * sizeof(double), w,
-                              eb::kStateFields, cudaMemcpyDeviceToHost, s->stream));
-    pos += static_cast<size_t>(c) * eb::kStateFields;
+  unsigned char* dev = s->d_upload + base_off;
+  const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(dev);
+  SV_CUDA(cudaMemcpyAsync(dev, s->upload.base + base_off, bytes, cudaMemcpyHostToDevice, s->stream));
+  SV_CUDA(eb::launch_rod_energy_list(drefs, static_cast<int64_t>(nr), s->stride, s->rod_start, s->rod_n,
+                                     s->state[s->cur], s->par, s->e1, s->stream));
+  SV_CUDA(eb::launch_rod_result(drefs, static_cast<int64_t>(nr), s->stride, s->state[s->cur], s->rod_start, s->rod_n,
+                                s->e0, s->e1, s->stream));
+  if (eb_status st = close_stage(s)) return st;
+  for (Request* r : batch) {
+    if (!r->event) SV_CUDA(cudaEventCreateWithFlags(&r->event, cudaEventDisableTiming));
+    SV_CUDA(cudaEventRecord(r->event, s->stream));
+    // bins and rod ids go back at once: the launches above run before any
+    // later use of them on this stream
+    for (size_t b = 0; b < r->bins.size(); ++b) {
+      if (r->bin_pair[b])
+        s->bins.give_pair(r->bins[b]);
+      else
+        s->bins.give_single(r->bins[b]);
+    }
+    s->rod_ids.release(r->rod0, static_cast<int64_t>(r->rods.size()));
+    r->state = kFinishing;
+    s->finishing.push_back(r);
   }
-  SV_CUDA(cudaMemcpyAsync(dst + pos, s->e0 + 5 * r.rod0, 5 * nr * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-  SV_CUDA(cudaMemcpyAsync(dst + pos + 5 * nr, s->e1 + 5 * r.rod0, 5 * nr * sizeof(double), cudaMemcpyDeviceToHost,
-                          s->stream));
-  if (!r.event) SV_CUDA(cudaEventCreateWithFlags(&r.event, cudaEventDisableTiming));
-  SV_CUDA(cudaEventRecord(r.event, s->stream));
-  // bins and rod ids go back at once: the copies above run before any later
-  // use of them on this stream
-  for (size_t b = 0; b < r.bins.size(); ++b) {
-    if (r.bin_pair[b])
-      s->bins.give_pair(r.bins[b]);
-    else
-      s->bins.give_single(r.bins[b]);
-  }
-  s->rod_ids.release(r.rod0, nr);
-  r.state = kFinishing;
-  s->finishing.push_back(&r);
   return EB_OK;
+}
+
+eb_status retire(eb_server* s, const std::vector<Request*>& done) {
+  std::vector<Request*> batch;
+  size_t refs = 0;
+  for (Request* r : done) {
+    const size_t nr = r->rods.size();
+    size_t slots = 0;
+    for (int32_t c : r->bin_count) slots += static_cast<size_t>(c);
+    const size_t bytes = (slots * eb::kStateFields + 10 * nr) * sizeof(double);
+    if (!batch.empty() && (refs + nr) * sizeof(eb::RodRef) > kUploadBytes / 2) {
+      if (eb_status st = retire_batch(s, batch)) return st;
+      batch.clear();
+      refs = 0;
+    }
+    while (!s->arena.alloc(bytes, &r->arena_off)) {
+      // the arena is full: enqueue what has its room, then wait for the
+      // oldest retirement and take it out
+      if (!batch.empty()) {
+        if (eb_status st = retire_batch(s, batch)) return st;
+        batch.clear();
+        refs = 0;
+      }
+      if (s->finishing.empty()) return fail(EB_ERR_OUT_OF_MEMORY, "request result larger than the host arena");
+      if (eb_status st = poll_events(s, true)) return st;
+    }
+    batch.push_back(r);
+    refs += nr;
+  }
+  return retire_batch(s, batch);
 }
 
 // Take a landed retirement out of the arena: energies, drift check, result.
@@ -589,23 +608,7 @@ void land(eb_server* s, Request& r) {
   r.e0 = E0;
   r.e1 = E1;
   r.escale = scale;
-  // result per rod in the local slot layout
-  r.result.clear();
-  r.result_off.assign(r.rods.size(), 0);
-  std::vector<size_t> bin_pos(r.bin_count.size(), 0);
-  size_t pos = 0;
-  for (size_t b = 0; b < r.bin_count.size(); ++b) {
-    bin_pos[b] = pos;
-    pos += static_cast<size_t>(r.bin_count[b]) * eb::kStateFields;
-  }
-  for (size_t k = 0; k < r.rods.size(); ++k) {
-    const int64_t W = r.rods[k].n_elements + 1, b = r.rod_bin[k], o = r.rod_off[k], c = r.bin_count[b];
-    r.result_off[k] = static_cast<int64_t>(r.result.size());
-    for (int f = 0; f < eb::kStateFields; ++f) {
-      const double* row = src + bin_pos[b] + static_cast<size_t>(f * c + o);
-      r.result.insert(r.result.end(), row, row + W);
-    }
-  }
+  r.result.assign(src, src + slots * eb::kStateFields);  // per rod, at its result_off
   s->arena.free_oldest();
   const bool drift_ok = finite && (E1 - E0) <= s->cfg.energy_tolerance * (scale > 0.0 ? scale : 1.0) &&
                        !(s->cfg.flags & EB_SERVER_FORCE_FALLBACK);
@@ -703,6 +706,7 @@ EB_API eb_status eb_server_create(const eb_server_config* config, eb_server** ou
   alloc(&s->e0, static_cast<size_t>(s->rod_cap) * 5 * sizeof(double));
   alloc(&s->e1, static_cast<size_t>(s->rod_cap) * 5 * sizeof(double));
   alloc(&s->status, sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->d_upload), kUploadBytes);
   for (int a = 0; a < 2; ++a)
     for (int b = 0; b < 2; ++b) {
       // one entry per bin, plus the padding entry of an odd count
@@ -750,9 +754,9 @@ EB_API eb_status eb_server_submit(eb_server* s, const eb_request* req, int64_t* 
   auto r = std::make_unique<Request>();
   r->rods.assign(req->rods, req->rods + req->n_rods);
   for (const auto& p : r->rods) {
-    eb::HostRodData check;  // the reference initializer's argument checks
+    eb::RodSpec check;  // the reference initializer's argument checks
     if (p.n_elements >= 2 && p.n_elements + 1 <= kPairSlots)
-      if (eb_status st = eb::host_straight_rod(p, check)) return st;
+      if (eb_status st = eb::straight_rod_spec(p, check)) return st;
   }
   for (const auto& p : r->rods) {
     if (p.n_elements < 2) return fail(EB_ERR_INVALID_ARGUMENT, "a rod needs at least 2 elements");
@@ -860,18 +864,15 @@ EB_API eb_status eb_server_tick(eb_server* s, int64_t* in_flight) {
     }
     if (s->launch_timed[parity]) SV_CUDA(cudaEventRecord(s->launch_t1[parity], s->stream));
     s->cur ^= 1;
-    std::vector<Request*> still;
+    std::vector<Request*> still, done;
     for (Request* r : s->active) {
       const int64_t steps = std::min<int64_t>(K, r->n_steps - r->steps_done);
       r->steps_done += steps;
       s->element_steps += static_cast<double>(steps) * static_cast<double>(r->elements);
-      if (r->steps_done >= r->n_steps) {
-        if (eb_status st = retire(s, *r)) return st;
-      } else {
-        still.push_back(r);
-      }
+      (r->steps_done >= r->n_steps ? done : still).push_back(r);
     }
     s->active.swap(still);
+    if (eb_status st = retire(s, done)) return st;
   }
   SV_CUDA(cudaEventRecord(s->tick_event[parity], s->stream));
   s->tick_pending[parity] = true;
