@@ -51,8 +51,8 @@
 // slots that carry them.
 //
 // Rod pairs (kPair) as in rod_block_fp64.cu: a rod of up to 1039 elements on
-// a cluster of two CTAs, neighbour reads across the split from the partner's
-// shared memory, both per-step barriers cluster barriers.
+// a cluster of two CTAs, the slots at the split copied to the partner's shared
+// memory, both per-step barriers cluster barriers.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
@@ -79,8 +79,8 @@ constexpr int kQRows = 5;  // double2 rows of the director
 enum MixedRowP : int {
   pA1 = 0,  // rest length, shear rigidity (3)
   pA2 = 1,  // inertia J (3), Voronoi rest length
-  pA3 = 2,  // rest curvature (3), -
-  pA4 = 3,  // bend rigidity (3), -
+  pA3 = 2,  // rest curvature (3), 1 / rest length
+  pA4 = 3,  // bend rigidity (3), 1 / Voronoi rest length
   pB1 = 4,  // J^-1 (3), mass
   pB2 = 5,  // damper rate nu_r, 1 - exp(-nu_t dt), explicit damping nu_f, nu_t
   pFE = 6,  // internal load (3), dilatation (exchanged)
@@ -91,12 +91,12 @@ enum MixedRowP : int {
 // bytes of shared memory a slot: 13 FP64 rows, 5 double2, 9 float4, two words
 constexpr int kMixedSlotBytes = dRowsD * 8 + kQRows * 16 + kRowsP * 16 + 8;
 
-template <int kCap>
+template <int kRow>
 struct MRows {
   double* d;
   double2* q;
   float4* p;
-  __device__ __forceinline__ double& ad(int r, int s) const { return d[r * kCap + s]; }
+  __device__ __forceinline__ double& ad(int r, int s) const { return d[r * kRow + s]; }
   __device__ __forceinline__ D3 d3(int r, int s) const { return {ad(r, s), ad(r + 1, s), ad(r + 2, s)}; }
   __device__ __forceinline__ void pd3(int r, int s, D3 v) const {
     ad(r, s) = v.x;
@@ -106,19 +106,19 @@ struct MRows {
   __device__ __forceinline__ void ldq(int s, double o[9]) const {
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const double2 v = q[k * kCap + s];
+      const double2 v = q[k * kRow + s];
       o[2 * k] = v.x;
       o[2 * k + 1] = v.y;
     }
-    o[8] = q[4 * kCap + s].x;
+    o[8] = q[4 * kRow + s].x;
   }
   __device__ __forceinline__ void stq(int s, const double o[9]) const {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) q[k * kCap + s] = make_double2(o[2 * k], o[2 * k + 1]);
-    q[4 * kCap + s] = make_double2(o[8], 0.0);
+    for (int k = 0; k < 4; ++k) q[k * kRow + s] = make_double2(o[2 * k], o[2 * k + 1]);
+    q[4 * kRow + s] = make_double2(o[8], 0.0);
   }
-  __device__ __forceinline__ float4 p4(int r, int s) const { return p[r * kCap + s]; }
-  __device__ __forceinline__ void sp4(int r, int s, float4 v) const { p[r * kCap + s] = v; }
+  __device__ __forceinline__ float4 p4(int r, int s) const { return p[r * kRow + s]; }
+  __device__ __forceinline__ void sp4(int r, int s, float4 v) const { p[r * kRow + s] = v; }
 };
 
 __device__ __forceinline__ F3 tof(D3 a) {
@@ -162,8 +162,8 @@ __device__ __forceinline__ float exp_small(float x) {
 }
 
 // x += c v; Q <- exp(-c [w]x) Q for element slots
-template <int kCap>
-__device__ __forceinline__ void drift(const MRows<kCap>& R, int s, uint32_t meta, double c, D3 v, D3 w) {
+template <int kRow>
+__device__ __forceinline__ void drift(const MRows<kRow>& R, int s, uint32_t meta, double c, D3 v, D3 w) {
   const D3 x = R.d3(dX, s);
   R.pd3(dX, s, D3{x.x + c * v.x, x.y + c * v.y, x.z + c * v.z});
   if (meta & kElem) {
@@ -176,8 +176,8 @@ __device__ __forceinline__ void drift(const MRows<kCap>& R, int s, uint32_t meta
 
 // the clamp's value constraint on a slot a clamp holds (hits: SlotHits):
 // the node's position and, where the slot holds an element, its directors
-template <int kCap>
-__device__ __forceinline__ void clamp_value(const MRows<kCap>& R, int s, uint32_t meta, uint32_t hits,
+template <int kRow>
+__device__ __forceinline__ void clamp_value(const MRows<kRow>& R, int s, uint32_t meta, uint32_t hits,
                                             const RodInfo& ri) {
   const double* tx = (hits & kHitClamp0) ? ri.clamp_x : ri.clamp2_x;
   const double* tq = (hits & kHitClamp0) ? ri.clamp_Q : ri.clamp2_Q;
@@ -189,40 +189,13 @@ __device__ __forceinline__ void clamp_value(const MRows<kCap>& R, int s, uint32_
   R.stq(s, q);
 }
 
-// Neighbour access for rod pairs: slot indices at or past `count` continue in
-// the partner's first slots (left half), indices below zero in the partner's
-// last `pcount` slots (right half).
-template <int kCap>
-struct MPair {
-  MRows<kCap> own, peer;
-  int count, pcount;
-  __device__ __forceinline__ const MRows<kCap>& rows(int& s) const {
-    if (s >= count) {
-      s -= count;
-      return peer;
-    }
-    if (s < 0) {
-      s += pcount;
-      return peer;
-    }
-    return own;
-  }
-  __device__ __forceinline__ D3 d3(int r, int s) const {
-    const MRows<kCap>& X = rows(s);
-    return X.d3(r, s);
-  }
-  __device__ __forceinline__ void ldq(int s, double o[9]) const {
-    const MRows<kCap>& X = rows(s);
-    X.ldq(s, o);
-  }
-  __device__ __forceinline__ float4 p4(int r, int s) const {
-    const MRows<kCap>& X = rows(s);
-    return X.p4(r, s);
-  }
-};
+// entries of a row: a CTA of a pair also holds copies of the partner's
+// neighbouring slots, one before its first slot and two after its last (see
+// rod_block_fp64.cu)
+template <int kCap, bool kPair>
+constexpr int mixed_row() { return kPair ? kCap + 4 : kCap; }
 
-// FP32 length of element s from its FP64 position difference (Rows: MRows,
-// or MPair for slots that may lie in a pair's partner)
+// FP32 length of element s from its FP64 position difference
 template <class Rows>
 __device__ __forceinline__ float element_length(const Rows& R, int s) {
   const F3 dxf = tof(R.d3(dX, s + 1) - R.d3(dX, s));
@@ -241,10 +214,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     rod_block_mixed_kernel(const StepArgs a, const int64_t* cta_start, int n_steps_launch, const ServeCta* serve,
                            const int32_t* gmap) {
   extern __shared__ __align__(128) double smem[];
-  double2* const qbase = reinterpret_cast<double2*>(smem + dRowsD * kCap);
-  float4* const pbase = reinterpret_cast<float4*>(qbase + kQRows * kCap);
-  const MRows<kCap> R{smem, qbase, pbase};
-  uint32_t* meta_s = reinterpret_cast<uint32_t*>(pbase + kRowsP * kCap);
+  constexpr int kRow = mixed_row<kCap, kPair>(), kShift = kPair ? 1 : 0;
+  double2* const qbase = reinterpret_cast<double2*>(smem + dRowsD * kRow);
+  float4* const pbase = reinterpret_cast<float4*>(qbase + kQRows * kRow);
+  const MRows<kRow> R{smem + kShift, qbase + kShift, pbase + kShift};
+  uint32_t* meta_s = reinterpret_cast<uint32_t*>(pbase + kRowsP * kRow);
   uint32_t* rflag_s = meta_s + kCap;
 
   const int tid = threadIdx.x;
@@ -270,26 +244,30 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   }
   if (n_steps <= 0) return;
   const int64_t S = a.stride;
-  // partner rows (its own rows for a single CTA) and cluster barriers
-  MPair<kCap> N{R, R, count, count};
-  bool paired = false;
+  // the partner's rows, at the place of this CTA's slot 0 (left half: past the
+  // end of the right half's left copy; right half: the left half's count)
+  MRows<kRow> peer = R;
+  bool paired = false, left = false;
   if constexpr (kPair) {
     const unsigned partner = blockIdx.x ^ 1u;
+    int pcount = 0;
     if constexpr (kServe) {
       const ServeCta& sc = serve[blockIdx.x];
       const ServeCta& o = serve[partner];
       paired = sc.pair != 0 && o.pair != 0 && sc.steps == o.steps;
-      if (paired) N.pcount = o.count;
+      pcount = o.count;
     } else {
       paired = true;
-      N.pcount = static_cast<int>(cta_start[partner + 1] - cta_start[partner]);
+      pcount = static_cast<int>(cta_start[partner + 1] - cta_start[partner]);
     }
     if (paired) {
       cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
       const unsigned pr = cl.block_rank() ^ 1u;
-      N.peer.d = cl.map_shared_rank(R.d, pr);
-      N.peer.q = cl.map_shared_rank(R.q, pr);
-      N.peer.p = cl.map_shared_rank(R.p, pr);
+      left = cl.block_rank() == 0;
+      const int at = left ? -count : pcount;
+      peer.d = cl.map_shared_rank(R.d, pr) + at;
+      peer.q = cl.map_shared_rank(R.q, pr) + at;
+      peer.p = cl.map_shared_rank(R.p, pr) + at;
     }
   }
   // orders a phase's writes before the next phase's neighbour reads
@@ -338,25 +316,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     auto pf = [&](int f) { return static_cast<float>(a.par[f * S + g]); };
     R.sp4(pA1, s, make_float4(pf(kL0), pf(kShear), pf(kShear + 1), pf(kShear + 2)));
     R.sp4(pA2, s, make_float4(pf(kJ), pf(kJ + 1), pf(kJ + 2), pf(kD0)));
-    R.sp4(pA3, s, make_float4(pf(kKap0), pf(kKap0 + 1), pf(kKap0 + 2), 0.f));
-    R.sp4(pA4, s, make_float4(pf(kBend), pf(kBend + 1), pf(kBend + 2), 0.f));
+    R.sp4(pA3, s, make_float4(pf(kKap0), pf(kKap0 + 1), pf(kKap0 + 2), static_cast<float>(il0)));
+    R.sp4(pA4, s, make_float4(pf(kBend), pf(kBend + 1), pf(kBend + 2), __frcp_rn(pf(kD0))));
     R.sp4(pB1, s, make_float4(pf(kJinv), pf(kJinv + 1), pf(kJinv + 2), pf(kMass)));
     R.sp4(pB2, s, make_float4(dr, static_cast<float>(1.0 - dtc), kDamped ? pf(kNuF) : 0.f,
                               kDamped ? pf(kNuT) : 0.f));
   }
-  __syncthreads();
+  sync_neighbours();
 
   const float dtf = static_cast<float>(dt);
   const F3 grav = {static_cast<float>(gvec[0]), static_cast<float>(gvec[1]), static_cast<float>(gvec[2])};
-
-  // ---- first half drift of the first step and the clamp's value constraint
-  for (int s = tid; s < count; s += kThreads) {
-    const uint32_t meta = meta_s[s];
-    drift(R, s, meta, hdt, R.d3(dV, s), R.d3(dW, s));
-    const uint32_t hits = rflag_s[s];
-    if (hits & (kHitClamp0 | kHitClamp1)) clamp_value(R, s, meta, hits, a.rods[meta >> kRodShift]);
-  }
-  sync_neighbours();
 
   // Two phases per step, one barrier after each.  Phase A: element s (strain,
   // internal load, element-local torque terms) and Voronoi s (curvature and
@@ -364,182 +333,244 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   // Phase B: loads, torques, kick, rate constraints, then the merged drift
   // (second half of this step and first half of the next; half on the last
   // step), the value constraint and, on the last step, the write-back.
-  for (int step = 0; step < n_steps; ++step) {
-    const bool last = step == n_steps - 1;
+  //
+  // A CTA of at most kThreads slots keeps a slot's angular velocity, which no
+  // neighbour reads, and what its phase A hands to its phase B in registers; a
+  // longer one keeps them in rows.
 
-    for (int s = tid; s < count; s += kThreads) {
-      const uint32_t meta = meta_s[s];
-      F3 f{0.f, 0.f, 0.f}, p{0.f, 0.f, 0.f}, mm{0.f, 0.f, 0.f};
-      float e = 1.f;
-      if (meta & kElem) {
-        const D3 dx = (kPair ? N.d3(dX, s + 1) : R.d3(dX, s + 1)) - R.d3(dX, s);
+  // mass of the next node of the rod (a pair's last slot reads its copy)
+  auto next_mass = [&](int s) -> float { return R.p4(pB1, s + 1).w; };
+  // positions, velocities and directors that the partner's slots read
+  auto publish = [&](int s) {
+    if (kPair && paired && !left && s < 2) {  // the left half's copies after its last slot
+      peer.pd3(dX, s, R.d3(dX, s));
+      peer.pd3(dV, s, R.d3(dV, s));
+      double q[9];
+      R.ldq(s, q);
+      peer.stq(s, q);
+    }
+  };
+  // phase A; wd: the slot's angular velocity; returns the load with the
+  // dilatation, and the torque terms in p
+  auto evaluate = [&](int s, uint32_t meta, D3 wd, F3& p) -> float4 {
+    F3 f{0.f, 0.f, 0.f}, mm{0.f, 0.f, 0.f};
+    p = F3{0.f, 0.f, 0.f};
+    float e = 1.f;
+    if (meta & kElem) {
+      const D3 dx = R.d3(dX, s + 1) - R.d3(dX, s);
+      double q[9];
+      R.ldq(s, q);
+      double qd[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) qd[k] = q[3 * k] * dx.x + q[3 * k + 1] * dx.y + q[3 * k + 2] * dx.z;
+      const double il0 = R.ad(dInvL0, s);
+      const F3 d = {static_cast<float>(qd[0] * il0 - R.ad(dSig0, s)),
+                    static_cast<float>(qd[1] * il0 - R.ad(dSig0 + 1, s)),
+                    static_cast<float>(qd[2] * il0 - R.ad(dSig0 + 2, s))};
+      const F3 dxf = tof(dx);
+      const float l2 = dot(dxf, dxf);
+      const float il = rsqrtf(l2);
+      const float l = l2 * il;
+      const F3 t = scale(dxf, il);
+      const float4 a1 = R.p4(pA1, s), a2 = R.p4(pA2, s), a3 = R.p4(pA3, s);
+      const float l0 = a1.x;
+      e = l * a3.w;
+      const float ie = l0 * il;
+      const F3 nl = {a1.y * d.x, a1.z * d.y, a1.w * d.z};
+      float qf[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) qf[k] = static_cast<float>(q[k]);
+      f = scale(mattranspvec(qf, nl), ie);
+      const F3 qt = matvec(qf, t);
+      const F3 w = tof(wd);
+      const F3 jwe = {a2.x * w.x * ie, a2.y * w.y * ie, a2.z * w.z * ie};
+      const F3 dv = tof(R.d3(dV, s + 1) - R.d3(dV, s));
+      const float rate = dot(t, dv) * il;
+      p = scale(cross(qt, nl), l0) + cross(jwe, w) + scale(jwe, rate);
+
+      if (meta & kVor) {
+        // With d_k the director rows of element s and dd_k = d_k(s+1) - d_k(s)
+        // (FP64 differences), the reference's skew terms are exactly
+        //   d3.d2' - d2.d3' = d3.dd2 - d2.dd3 (and cyclic), since d3.d2 = d2.d3,
+        // and 1 - cos(theta) = 1.5 - tr/2 = |dd|^2/4 for unit rows (their
+        // norms stay within 1e-14 of one, below the reference's 1e-10 shift);
+        // both forms are free of the cancellation of the original products.
+        double qn[9];
+        R.ldq(s + 1, qn);
+        float dd[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) dd[k] = static_cast<float>(qn[k] - q[k]);
+        float sq = 0.f;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) sq += dd[k] * dd[k];
+        const float y = 0.25f * sq + 1e-10f;
+        float ratio;  // theta / sin(theta), theta = acos(1 - y)
+        if (y < 0.25f) {
+          // its Taylor series in y = 1 - cos(theta) through y^7 (the
+          // first omitted term is below 2e-8 for y < 0.25, under FP32's
+          // rounding), which covers relative rotations up to 0.72 rad a
+          // Voronoi point without the arcsine
+          ratio = 1.f + y * (1.f / 3.f + y * (2.f / 15.f + y * (2.f / 35.f + y * (8.f / 315.f +
+                  y * (8.f / 693.f + y * (16.f / 3003.f + y * (16.f / 6435.f)))))));
+        } else {
+          ratio = 2.f * asinf(sqrtf(0.5f * y)) * rsqrtf(y * (2.f - y));
+        }
+        const float D0 = a2.w;
+        const float4 a4 = R.p4(pA4, s);
+        const float st = 0.5f * ratio * a4.w;
+        const F3 d1{qf[0], qf[1], qf[2]}, d2{qf[3], qf[4], qf[5]}, d3{qf[6], qf[7], qf[8]};
+        const F3 e1{dd[0], dd[1], dd[2]}, e2{dd[3], dd[4], dd[5]}, e3{dd[6], dd[7], dd[8]};
+        const F3 skew = {dot(d3, e2) - dot(d2, e3), dot(d1, e3) - dot(d3, e1), dot(d2, e1) - dot(d1, e2)};
+        const F3 kappa = scale(skew, st);
+        // 1 / eps^3 with eps = D / D0, D the mean length of elements s, s + 1
+        const float ieps =
+            __fdividef(D0, 0.5f * (l + element_length(R, s + 1)));
+        const float ic = ieps * ieps * ieps;
+        const F3 dk = kappa - xyz(a3);
+        const F3 B = xyz(a4);
+        const F3 tau = {B.x * dk.x, B.y * dk.y, B.z * dk.z};
+        // the couple's two parts: G = tau / eps^3 (differenced) and
+        // H = (kappa x tau) D0 / eps^3 (averaged) enter torque s as
+        // (G_s + H_s / 2) - (G_{s-1} - H_{s-1} / 2)
+        const F3 gg = scale(tau, ic);
+        const F3 hh = scale(cross(kappa, tau), 0.5f * ic * D0);
+        p = p + gg + hh;
+        mm = gg - hh;
+      }
+    }
+    const float4 fe = make_float4(f.x, f.y, f.z, e), m4 = make_float4(mm.x, mm.y, mm.z, 0.f);
+    R.sp4(pFE, s, fe);
+    R.sp4(pMM, s, m4);
+    if (kPair && paired && left && s == count - 1) {  // the right half's copy before its first slot
+      peer.sp4(pFE, s, fe);
+      peer.sp4(pMM, s, m4);
+    }
+    return fe;
+  };
+  // phase B of slot s (rf: its SlotHits; w: its angular velocity)
+  auto kick = [&](int s, uint32_t meta, uint32_t rf, float4 fe, F3 p, D3& w, bool last) {
+    const bool first = (meta & kFirst) != 0;
+    const float4 b1 = R.p4(pB1, s);
+    const float m = b1.w;
+    D3 v = R.d3(dV, s);
+    F3 F = xyz(fe);
+    if (!first) F = F - xyz(R.p4(pFE, s - 1));
+    float4 b2 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kDamped || (rf & kHitDamper)) b2 = R.p4(pB2, s);
+    if (kDamped) {
+      const float cf = m * b2.z;
+      const F3 vf = tof(v);
+      F = {F.x - cf * vf.x, F.y - cf * vf.y, F.z - cf * vf.z};
+    }
+    if (flags & kSimGravity) F = F + F3{grav.x * m, grav.y * m, grav.z * m};
+    const float im = __frcp_rn(m);
+    v = {v.x + dt * static_cast<double>(F.x * im), v.y + dt * static_cast<double>(F.y * im),
+         v.z + dt * static_cast<double>(F.z * im)};
+    if (meta & kElem) {
+      const float e = fe.w;
+      F3 T = p;
+      if (!first) T = T - xyz(R.p4(pMM, s - 1));
+      const float mn = (kDamped || (rf & kHitDamper)) ? next_mass(s) : 0.f;
+      if (kDamped) {
+        const float ct = 0.5f * (m + mn) * b2.w;
+        const F3 wf = tof(w);
+        T = {T.x - ct * wf.x, T.y - ct * wf.y, T.z - ct * wf.z};
+      }
+      if (rf & kHitTorque) {
+        const RodInfo& ri = a.rods[meta >> kRodShift];
         double q[9];
         R.ldq(s, q);
-        double qd[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) qd[k] = q[3 * k] * dx.x + q[3 * k + 1] * dx.y + q[3 * k + 2] * dx.z;
-        const double il0 = R.ad(dInvL0, s);
-        const F3 d = {static_cast<float>(qd[0] * il0 - R.ad(dSig0, s)),
-                      static_cast<float>(qd[1] * il0 - R.ad(dSig0 + 1, s)),
-                      static_cast<float>(qd[2] * il0 - R.ad(dSig0 + 2, s))};
-        const F3 dxf = tof(dx);
-        const float l2 = dot(dxf, dxf);
-        const float il = rsqrtf(l2);
-        const float l = l2 * il;
-        const F3 t = scale(dxf, il);
-        const float4 a1 = R.p4(pA1, s), a2 = R.p4(pA2, s);
-        const float l0 = a1.x;
-        e = l * static_cast<float>(il0);
-        const float ie = l0 * il;
-        const F3 nl = {a1.y * d.x, a1.z * d.y, a1.w * d.z};
         float qf[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) qf[k] = static_cast<float>(q[k]);
-        f = scale(mattranspvec(qf, nl), ie);
-        const F3 qt = matvec(qf, t);
-        const F3 w = tof(R.d3(dW, s));
-        const F3 jwe = {a2.x * w.x * ie, a2.y * w.y * ie, a2.z * w.z * ie};
-        const F3 dv = tof((kPair ? N.d3(dV, s + 1) : R.d3(dV, s + 1)) - R.d3(dV, s));
-        const float rate = dot(t, dv) * il;
-        p = scale(cross(qt, nl), l0) + cross(jwe, w) + scale(jwe, rate);
-
-        if (meta & kVor) {
-          // With d_k the director rows of element s and dd_k = d_k(s+1) - d_k(s)
-          // (FP64 differences), the reference's skew terms are exactly
-          //   d3.d2' - d2.d3' = d3.dd2 - d2.dd3 (and cyclic), since d3.d2 = d2.d3,
-          // and 1 - cos(theta) = 1.5 - tr/2 = |dd|^2/4 for unit rows (their
-          // norms stay within 1e-14 of one, below the reference's 1e-10 shift);
-          // both forms are free of the cancellation of the original products.
-          double qn[9];
-          if constexpr (kPair) N.ldq(s + 1, qn);
-          else R.ldq(s + 1, qn);
-          float dd[9];
-#pragma unroll
-          for (int k = 0; k < 9; ++k) dd[k] = static_cast<float>(qn[k] - q[k]);
-          float sq = 0.f;
-#pragma unroll
-          for (int k = 0; k < 9; ++k) sq += dd[k] * dd[k];
-          const float y = 0.25f * sq + 1e-10f;
-          float ratio;  // theta / sin(theta), theta = acos(1 - y)
-          if (y < 0.25f) {
-            // its Taylor series in y = 1 - cos(theta) through y^7 (the
-            // first omitted term is below 2e-8 for y < 0.25, under FP32's
-            // rounding), which covers relative rotations up to 0.72 rad a
-            // Voronoi point without the arcsine
-            ratio = 1.f + y * (1.f / 3.f + y * (2.f / 15.f + y * (2.f / 35.f + y * (8.f / 315.f +
-                    y * (8.f / 693.f + y * (16.f / 3003.f + y * (16.f / 6435.f)))))));
-          } else {
-            ratio = 2.f * asinf(sqrtf(0.5f * y)) * rsqrtf(y * (2.f - y));
-          }
-          const float D0 = a2.w;
-          const float st = 0.5f * ratio * __frcp_rn(D0);
-          const F3 d1{qf[0], qf[1], qf[2]}, d2{qf[3], qf[4], qf[5]}, d3{qf[6], qf[7], qf[8]};
-          const F3 e1{dd[0], dd[1], dd[2]}, e2{dd[3], dd[4], dd[5]}, e3{dd[6], dd[7], dd[8]};
-          const F3 skew = {dot(d3, e2) - dot(d2, e3), dot(d1, e3) - dot(d3, e1), dot(d2, e1) - dot(d1, e2)};
-          const F3 kappa = scale(skew, st);
-          // 1 / eps^3 with eps = D / D0, D the mean length of elements s, s + 1
-          const float ieps =
-              __fdividef(D0, 0.5f * (l + (kPair ? element_length(N, s + 1) : element_length(R, s + 1))));
-          const float ic = ieps * ieps * ieps;
-          const F3 dk = kappa - xyz(R.p4(pA3, s));
-          const F3 B = xyz(R.p4(pA4, s));
-          const F3 tau = {B.x * dk.x, B.y * dk.y, B.z * dk.z};
-          // the couple's two parts: G = tau / eps^3 (differenced) and
-          // H = (kappa x tau) D0 / eps^3 (averaged) enter torque s as
-          // (G_s + H_s / 2) - (G_{s-1} - H_{s-1} / 2)
-          const F3 gg = scale(tau, ic);
-          const F3 hh = scale(cross(kappa, tau), 0.5f * ic * D0);
-          p = p + gg + hh;
-          mm = gg - hh;
-        }
+        T = T + matvec(qf, F3{static_cast<float>(ri.end_torque[0]), static_cast<float>(ri.end_torque[1]),
+                              static_cast<float>(ri.end_torque[2])});
       }
-      R.sp4(pFE, s, make_float4(f.x, f.y, f.z, e));
+      const F3 ji = xyz(b1);
+      w = {w.x + dt * static_cast<double>(ji.x * T.x * e), w.y + dt * static_cast<double>(ji.y * T.y * e),
+           w.z + dt * static_cast<double>(ji.z * T.z * e)};
+      if (rf & kHitDamper) {
+        float em = 0.5f * (m + mn);
+        if (first) em += 0.5f * m;
+        if (meta & kLastElem) em += 0.5f * mn;
+        const float y = -b2.x * em * dtf * e;
+        // (a circular cross section: one factor for both bending directions)
+        const double ex = static_cast<double>(exp_small(y * ji.x));
+        w = {w.x * ex, w.y * (ji.y == ji.x ? ex : static_cast<double>(exp_small(y * ji.y))),
+             w.z * static_cast<double>(exp_small(y * ji.z))};
+      }
+    }
+    const bool clamped = (rf & (kHitClamp0 | kHitClamp1)) != 0;
+    if (clamped) {
+      v = D3{0.0, 0.0, 0.0};
+      w = D3{0.0, 0.0, 0.0};
+    }
+    if (rf & kHitDamper) v = scale(v, 1.0 - static_cast<double>(b2.y));
+    R.pd3(dV, s, v);
+    drift(R, s, meta, last ? hdt : dt, v, w);
+    if (clamped) clamp_value(R, s, meta, rf, a.rods[meta >> kRodShift]);
+    if (!last) publish(s);
+  };
+  auto write_back = [&](int s, uint32_t meta, D3 w) {
+    const int64_t g = kGather ? static_cast<int64_t>(gmap[g0 + s]) : g0 + s;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      a.out[(kStX + k) * S + g] = R.ad(dX + k, s);
+      a.out[(kStV + k) * S + g] = R.ad(dV + k, s);
+    }
+    if (meta & kElem) {
+      double q[9];
+      R.ldq(s, q);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) a.out[(kStQ + k) * S + g] = q[k];
+      a.out[kStW * S + g] = w.x;
+      a.out[(kStW + 1) * S + g] = w.y;
+      a.out[(kStW + 2) * S + g] = w.z;
+    }
+  };
+
+  // ---- first half drift of the first step and the clamp's value constraint
+  for (int s = tid; s < count; s += kThreads) {
+    const uint32_t meta = meta_s[s];
+    drift(R, s, meta, hdt, R.d3(dV, s), R.d3(dW, s));
+    const uint32_t hits = rflag_s[s];
+    if (hits & (kHitClamp0 | kHitClamp1)) clamp_value(R, s, meta, hits, a.rods[meta >> kRodShift]);
+    publish(s);
+    if (kPair && paired && !left && s < 2) peer.sp4(pB1, s, R.p4(pB1, s));
+  }
+  sync_neighbours();
+
+  if (count <= kThreads) {
+    const bool on = tid < count;
+    const uint32_t meta = on ? meta_s[tid] : 0u, rf = on ? rflag_s[tid] : 0u;
+    D3 w{0.0, 0.0, 0.0};
+    if (on && (meta & kElem)) w = R.d3(dW, tid);
+    float4 fe = make_float4(0.f, 0.f, 0.f, 1.f);
+    F3 p{0.f, 0.f, 0.f};
+    for (int step = 0; step < n_steps; ++step) {
+      if (on) fe = evaluate(tid, meta, w, p);
+      sync_neighbours();
+      if (on) kick(tid, meta, rf, fe, p, w, step == n_steps - 1);
+      sync_neighbours();
+    }
+    if (on) write_back(tid, meta, w);
+    return;
+  }
+  for (int step = 0; step < n_steps; ++step) {
+    const bool last = step == n_steps - 1;
+    for (int s = tid; s < count; s += kThreads) {
+      F3 p;
+      evaluate(s, meta_s[s], R.d3(dW, s), p);
       R.sp4(pPP, s, make_float4(p.x, p.y, p.z, 0.f));
-      R.sp4(pMM, s, make_float4(mm.x, mm.y, mm.z, 0.f));
     }
     sync_neighbours();
-
     for (int s = tid; s < count; s += kThreads) {
       const uint32_t meta = meta_s[s];
-      const bool first = (meta & kFirst) != 0;
-      const float4 b1 = R.p4(pB1, s);
-      const float m = b1.w;
-      D3 v = R.d3(dV, s);
-      const float4 fe = R.p4(pFE, s);
-      F3 F = xyz(fe);
-      if (!first) F = F - xyz(kPair ? N.p4(pFE, s - 1) : R.p4(pFE, s - 1));
-      const uint32_t rf = rflag_s[s];
-      float4 b2 = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (kDamped || (rf & kHitDamper)) b2 = R.p4(pB2, s);
-      if (kDamped) {
-        const float cf = m * b2.z;
-        const F3 vf = tof(v);
-        F = {F.x - cf * vf.x, F.y - cf * vf.y, F.z - cf * vf.z};
-      }
-      if (flags & kSimGravity) F = F + F3{grav.x * m, grav.y * m, grav.z * m};
-      const float im = __frcp_rn(m);
-      v = {v.x + dt * static_cast<double>(F.x * im), v.y + dt * static_cast<double>(F.y * im),
-           v.z + dt * static_cast<double>(F.z * im)};
       D3 w{0.0, 0.0, 0.0};
-      if (meta & kElem) {
-        const float e = fe.w;
-        w = R.d3(dW, s);
-        F3 T = xyz(R.p4(pPP, s));
-        if (!first) T = T - xyz(kPair ? N.p4(pMM, s - 1) : R.p4(pMM, s - 1));
-        const float mn = (kDamped || (rf & kHitDamper)) ? (kPair ? N.p4(pB1, s + 1) : R.p4(pB1, s + 1)).w : 0.f;
-        if (kDamped) {
-          const float ct = 0.5f * (m + mn) * b2.w;
-          const F3 wf = tof(w);
-          T = {T.x - ct * wf.x, T.y - ct * wf.y, T.z - ct * wf.z};
-        }
-        if (rf & kHitTorque) {
-          const RodInfo& ri = a.rods[meta >> kRodShift];
-          double q[9];
-          R.ldq(s, q);
-          float qf[9];
-#pragma unroll
-          for (int k = 0; k < 9; ++k) qf[k] = static_cast<float>(q[k]);
-          T = T + matvec(qf, F3{static_cast<float>(ri.end_torque[0]), static_cast<float>(ri.end_torque[1]),
-                                static_cast<float>(ri.end_torque[2])});
-        }
-        const F3 ji = xyz(b1);
-        w = {w.x + dt * static_cast<double>(ji.x * T.x * e), w.y + dt * static_cast<double>(ji.y * T.y * e),
-             w.z + dt * static_cast<double>(ji.z * T.z * e)};
-        if (rf & kHitDamper) {
-          float em = 0.5f * (m + mn);
-          if (first) em += 0.5f * m;
-          if (meta & kLastElem) em += 0.5f * mn;
-          const float y = -b2.x * em * dtf * e;
-          w = {w.x * static_cast<double>(exp_small(y * ji.x)), w.y * static_cast<double>(exp_small(y * ji.y)),
-               w.z * static_cast<double>(exp_small(y * ji.z))};
-        }
-      }
-      const bool clamped = (rf & (kHitClamp0 | kHitClamp1)) != 0;
-      if (clamped) {
-        v = D3{0.0, 0.0, 0.0};
-        w = D3{0.0, 0.0, 0.0};
-      }
-      if (rf & kHitDamper) v = scale(v, 1.0 - static_cast<double>(b2.y));
-      R.pd3(dV, s, v);
+      if (meta & kElem) w = R.d3(dW, s);
+      kick(s, meta, rflag_s[s], R.p4(pFE, s), xyz(R.p4(pPP, s)), w, last);
       if (meta & kElem) R.pd3(dW, s, w);
-      drift(R, s, meta, last ? hdt : dt, v, w);
-      if (clamped) clamp_value(R, s, meta, rf, a.rods[meta >> kRodShift]);
-      if (last) {
-        const int64_t g = kGather ? static_cast<int64_t>(gmap[g0 + s]) : g0 + s;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          a.out[(kStX + k) * S + g] = R.ad(dX + k, s);
-          a.out[(kStV + k) * S + g] = R.ad(dV + k, s);
-        }
-        if (meta & kElem) {
-          double q[9];
-          R.ldq(s, q);
-#pragma unroll
-          for (int k = 0; k < 9; ++k) a.out[(kStQ + k) * S + g] = q[k];
-#pragma unroll
-          for (int k = 0; k < 3; ++k) a.out[(kStW + k) * S + g] = R.ad(dW + k, s);
-        }
-      }
+      if (last) write_back(s, meta, w);
     }
     sync_neighbours();
   }
@@ -548,7 +579,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 template <int kCap, int kThreads, int kMinBlocks, bool kServe = false, bool kGather = false, bool kPair = false>
 cudaError_t launch_mixed_cfg(const StepArgs& args, const int64_t* cta_start, int n_ctas, int n_steps, bool damped,
                              cudaStream_t stream, const ServeCta* serve = nullptr, const int32_t* gmap = nullptr) {
-  const size_t bytes = size_t(kMixedSlotBytes) * kCap;
+  const size_t bytes = size_t(kMixedSlotBytes - 8) * mixed_row<kCap, kPair>() + size_t(kCap) * 8;
   auto go = [&](auto kern) -> cudaError_t {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
     if (e != cudaSuccess) return e;
