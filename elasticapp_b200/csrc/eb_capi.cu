@@ -851,8 +851,9 @@ static eb_status batch_copy(eb_sim* s, int32_t field, int32_t layout, double* ho
     } else {
       EB_CUDA(cudaMemcpy2DAsync(host, w, base, pitch, w, fi.ncomp, cudaMemcpyDeviceToHost, s->stream));
     }
+    if (!to_device) return check_device_status(s);  // which waits for the stream
     EB_CUDA(cudaStreamSynchronize(s->stream));
-    return to_device ? EB_OK : check_device_status(s);
+    return EB_OK;
   }
   if (layout != EB_LAYOUT_PER_ROD) return fail(EB_ERR_INVALID_ARGUMENT, "unknown layout");
   int64_t total = 0;
@@ -2114,17 +2115,39 @@ EB_API eb_status eb_step_host_state(eb_sim* s, double* time, double dt, int64_t 
     overlap = !s->xgroups.empty();
   }
   if (!overlap) {
-    for (int f = 0; f < 4; ++f)
-      if (in[f])
-        if (eb_status st = batch_copy(s, kExchangeFields[f], EB_LAYOUT_SLOTS, const_cast<double*>(in[f]),
-                                      kFields[kExchangeFields[f]].ncomp * s->n_slots, true))
-          return st;
-    if (eb_status st = eb_step(s, time, dt, n_steps)) return st;
-    for (int f = 0; f < 4; ++f)
-      if (out[f])
-        if (eb_status st = batch_copy(s, kExchangeFields[f], EB_LAYOUT_SLOTS, out[f],
-                                      kFields[kExchangeFields[f]].ncomp * s->n_slots, false))
-          return st;
+    // every copy is queued on the stream, and the host waits once, at the end
+    // (waiting for each field and each status word took 70 of the 279 us that
+    // 32 one-step calls of a 100-element rod and the read of its state take)
+    const size_t w = static_cast<size_t>(s->n_slots) * sizeof(double);
+    const size_t dev_pitch = static_cast<size_t>(s->stride) * sizeof(double);
+    bool any_in = false;
+    auto copies = [&]() -> eb_status {
+      for (int f = 0; f < 4; ++f) {
+        if (!in[f]) continue;
+        any_in = true;
+        const FieldInfo& fi = kFields[kExchangeFields[f]];
+        double* base = s->d_state[s->cur] + fi.offset * s->stride;
+        EB_CUDA(cudaMemcpy2DAsync(base, dev_pitch, in[f], w, w, fi.ncomp, cudaMemcpyHostToDevice, s->stream));
+        EB_CUDA(cudaMemcpy2DAsync(s->d_state[s->cur ^ 1] + fi.offset * s->stride, dev_pitch, base, dev_pitch, w,
+                                  fi.ncomp, cudaMemcpyDeviceToDevice, s->stream));
+      }
+      if (eb_status st = eb_step(s, time, dt, n_steps)) return st;
+      for (int f = 0; f < 4; ++f) {
+        if (!out[f]) continue;
+        const FieldInfo& fi = kFields[kExchangeFields[f]];
+        EB_CUDA(cudaMemcpy2DAsync(out[f], w, s->d_state[s->cur] + fi.offset * s->stride, dev_pitch, w, fi.ncomp,
+                                  cudaMemcpyDeviceToHost, s->stream));
+      }
+      return EB_OK;
+    };
+    const eb_status st = copies();
+    // the caller's arrays are its own again on return, after an error too
+    if (st != EB_OK) {
+      cudaStreamSynchronize(s->stream);
+      return st;
+    }
+    if (any_out) return check_device_status(s);
+    if (any_in) EB_CUDA(cudaStreamSynchronize(s->stream));
     return EB_OK;
   }
   if (eb_status st = damper_for_dt(s, dt)) return st;
