@@ -151,11 +151,21 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
     const double* v = a.state + kStV * S;
     const double* w = a.state + kStW * S;
     const double c = a.half_dt;
+    // everything the capsule is made of is asked for before anything is
+    // written (a load after a store waits for it)
+    const uint32_t meta = a.meta[s];
+    const D3 xa = ld3(x, S, s), xb = ld3(x, S, s + 1), va = ld3(v, S, s), vb = ld3(v, S, s + 1), om = ld3(w, S, s);
+    const double l0 = a.par[kL0 * S + s], volume = a.par[kVol * S + s];
+    const double m0 = a.par[kMass * S + s], m1 = a.par[kMass * S + s + 1];
+    // the bucket the capsule was filed in last time holds nothing any more
+    // (those of its capsules all write the same; a bucket no capsule was
+    // filed in is empty already)
+    const uint32_t old = a.bucket[s];
+    if (old < a.max_cells) a.cell[old] = make_int2(0, 0);
     // positions after the first half drift (PositionVerlet.hpp:60-69) and
     // the clamp's value constraint
-    D3 x0 = {x[s] + c * v[s], x[S + s] + c * v[S + s], x[2 * S + s] + c * v[2 * S + s]};
-    D3 x1 = {x[s + 1] + c * v[s + 1], x[S + s + 1] + c * v[S + s + 1], x[2 * S + s + 1] + c * v[2 * S + s + 1]};
-    const uint32_t meta = a.meta[s];
+    D3 x0 = {xa.x + c * va.x, xa.y + c * va.y, xa.z + c * va.z};
+    D3 x1 = {xb.x + c * vb.x, xb.y + c * vb.y, xb.z + c * vb.z};
     // the far node of the next element of the rod
     const bool joint = (meta & kVor) != 0;
     D3 x2 = x1;
@@ -182,7 +192,6 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
       a.plain_joint[s] = joint && l2 > 1e-6 && n2 > 1e-6 && l2 < 1e8 && n2 < 1e8 && along > 0.0 &&
                          along * along > 0.01 * (l2 * n2) && fabs(x1.x) < 1e6 && fabs(x1.y) < 1e6 && fabs(x1.z) < 1e6;
     }
-    const double l0 = a.par[kL0 * S + s], volume = a.par[kVol * S + s];
     D3 t;
     double area;  // volume / (pi l)
     if (ordinary(l)) {
@@ -207,12 +216,9 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
       v2 = cross(v3, v1);
     }
     const D3 r0 = normalize3(v2), r1 = normalize3(v3), r2 = v1;
-    const double m0 = a.par[kMass * S + s], m1 = a.par[kMass * S + s + 1];
-    const D3 va = ld3(v, S, s), vb = ld3(v, S, s + 1);
     const D3 num = mul3(m0, va) + mul3(m1, vb);
     const double den = m0 + m1;
     const D3 vel = quotient3(num, den);
-    const D3 om = ld3(w, S, s);
     const D3 ww = {r0.x * om.x + r1.x * om.y + r2.x * om.z, r0.y * om.x + r1.y * om.y + r2.y * om.z,
                    r0.z * om.x + r1.z * om.y + r2.z * om.z};
     // the narrow phase writes only the capsules it evaluates
@@ -384,42 +390,30 @@ __global__ void __launch_bounds__(kThreads) cell_kernel(const ContactArgs a) {
   a.bucket[s] = b;
   // the capsule's rank in its bucket, kept in its pair count until the
   // scatter has filed it (the pair search then writes the count)
-  a.pair_count[s] = atomicAdd(a.bucket_count + b, 1);
+  a.pair_count[s] = atomicAdd(&a.cell[b].x, 1);
 }
 
-// The buckets' ranges of entries, in whatever order the CTAs come: a CTA
-// scans the counts of its buckets and takes their entries with one atomic.
-// (A scan of the whole table in bucket order took three launches, 24 us for
-// two million buckets against 8 us; no reader needs the order.)  The counts
-// go back to zero for the next evaluation.
-constexpr int kRangeItems = 8;
-
+// The buckets' first entries, in whatever order the CTAs come: the capsule of
+// rank 0 stands for its bucket, and a CTA scans the counts of its buckets and
+// takes their entries with one atomic.  (No reader needs the buckets in order,
+// and only those in use are looked at: a pass over every bucket, which also
+// set the counts back to zero, took 22 us for four million of them, this one
+// 9 us for the half million capsules in them.)
 __global__ void __launch_bounds__(kThreads) range_kernel(const ContactArgs a) {
   grid_dependency_launch();
   grid_dependency_wait();
-  // buckets in use: the hash table's or the dense grid's cells (max_cells, a
-  // power of two of at least 1024, holds either)
-  const ContactGrid& g = *a.grid;
-  const int64_t used = g.dense ? static_cast<int64_t>(g.slab) * (g.last[2] - g.first[2] + 1)
-                               : static_cast<int64_t>(a.table_mask) + 1;
-  const int64_t first = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) * kRangeItems;
-  if (static_cast<int64_t>(blockIdx.x) * kThreads * kRangeItems >= used) return;
-  const bool on = first < a.max_cells;
-  int32_t n[kRangeItems] = {0, 0, 0, 0, 0, 0, 0, 0};
-  int4* counts = reinterpret_cast<int4*>(a.bucket_count + first);
-  if (on) {
-    const int4 c0 = counts[0], c1 = counts[1];
-    n[0] = c0.x, n[1] = c0.y, n[2] = c0.z, n[3] = c0.w;
-    n[4] = c1.x, n[5] = c1.y, n[6] = c1.z, n[7] = c1.w;
-    counts[0] = counts[1] = make_int4(0, 0, 0, 0);
+  const int64_t s = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;
+  int2* cell = nullptr;
+  if (s < a.n_slots) {
+    const int32_t mat = a.cap_material[s], rank = a.pair_count[s];
+    const uint32_t b = a.bucket[s];
+    if (mat >= 0 && rank == 0 && b < a.max_cells) cell = a.cell + b;  // (past the last bucket: not filed)
   }
-  int32_t sum = 0;
-#pragma unroll
-  for (int i = 0; i < kRangeItems; ++i) sum += n[i];
+  const int32_t n = cell ? cell->x : 0;
   __shared__ int32_t warp_sum[kThreads / 32];
   __shared__ int32_t base;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int32_t x = sum;
+  int32_t x = n;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
     const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
@@ -437,15 +431,7 @@ __global__ void __launch_bounds__(kThreads) range_kernel(const ContactArgs a) {
     base = total ? atomicAdd(&a.grid->filed, total) : 0;
   }
   __syncthreads();
-  if (!on) return;
-  int32_t run = base + warp_sum[wid] + x - sum;
-  int4* out = reinterpret_cast<int4*>(a.bucket_range + first);
-#pragma unroll
-  for (int i = 0; i < kRangeItems; i += 2) {
-    const int32_t mid = run + n[i], end = mid + n[i + 1];
-    out[i / 2] = make_int4(run, mid, mid, end);
-    run = end;
-  }
+  if (cell) cell->y = base + warp_sum[wid] + x - n;
 }
 
 __global__ void __launch_bounds__(kThreads) scatter_kernel(const ContactArgs a) {
@@ -458,11 +444,12 @@ __global__ void __launch_bounds__(kThreads) scatter_kernel(const ContactArgs a) 
     a.grid->scanned = 0;
     for (int d = 0; d < 3; ++d) a.grid->top[d] = a.grid->bottom[d] = 0u;
   }
-  if (s >= a.n_slots || a.cap_material[s] < 0) return;
+  if (s >= a.n_slots) return;
   const int64_t S = a.stride;
+  const int32_t mat = a.cap_material[s], rank = a.pair_count[s];  // the rank the cell kernel took
   const uint32_t b = a.bucket[s];
-  if (b >= a.max_cells) return;  // excluded (not finite)
-  const int32_t pos = a.bucket_range[b].x + a.pair_count[s];  // the rank the cell kernel took
+  if (mat < 0 || b >= a.max_cells) return;  // no capsule, or excluded (not finite)
+  const int32_t pos = a.cell[b].y + rank;
   if (pos < 0 || pos >= a.n_caps) {  // cannot happen with consistent counts; never write out of range
     atomicOr(a.status, kStatusContactIndex);
     return;
@@ -569,17 +556,17 @@ __device__ __forceinline__ uint32_t search_one(const ContactArgs& a, const Conta
   bool live = false;
   int32_t cx = c0[0], cy = c0[1], cz = c0[2];
   bool more = c0[0] <= c1[0] && c0[1] <= c1[1] && c0[2] <= c1[2];
-  // the ranges of cells cx and cx + 1 of the row
+  // the counts and first entries of cells cx and cx + 1 of the row
   int2 ra = make_int2(0, 0), rb = make_int2(0, 0);
   auto fetch = [&]() {
-    ra = a.bucket_range[bucket_of(g, kDense, a.table_mask, cx, cy, cz)];
-    rb = cx < c1[0] ? a.bucket_range[bucket_of(g, kDense, a.table_mask, cx + 1, cy, cz)] : make_int2(0, 0);
+    ra = a.cell[bucket_of(g, kDense, a.table_mask, cx, cy, cz)];
+    rb = cx < c1[0] ? a.cell[bucket_of(g, kDense, a.table_mask, cx + 1, cy, cz)] : make_int2(0, 0);
   };
   if (more) fetch();
   while (more) {
     const int32_t hx = cx, hy = cy, hz = cz;
-    const int32_t a0 = max(ra.x, 0), na = max(min(ra.y, n_caps) - a0, 0);
-    const int32_t b0 = max(rb.x, 0), n = na + max(min(rb.y, n_caps) - b0, 0);
+    const int32_t a0 = max(ra.y, 0), na = max(min(ra.x, n_caps - a0), 0);
+    const int32_t b0 = max(rb.y, 0), n = na + max(min(rb.x, n_caps - b0), 0);
     cx += 2;
     if (cx > c1[0]) {
       cx = c0[0];
@@ -916,11 +903,10 @@ __global__ void __launch_bounds__(kForceThreads, kForceCtasPerSm) force_kernel(c
 cudaError_t launch_contact(const ContactArgs& a, cudaStream_t stream, int64_t* launches) {
   if (a.n_slots <= 0) return cudaSuccess;
   const unsigned gs = static_cast<unsigned>((a.n_slots + kThreads - 1) / kThreads);
-  // the largest box extent and the bucket counts are zero here: allocated
-  // zeroed, the extent set back to zero by the scatter once the cell kernel
-  // has used it, and each count by the range kernel as it reads it; the cell
-  // kernel zeroes the running totals
-  const int64_t table = a.max_cells;
+  // the largest box extent and the bucket counts are zero when they are added
+  // to: allocated zeroed, the extent set back to zero by the scatter once the
+  // cell kernel has used it, and each count by the next evaluation's capsule
+  // kernel; the cell kernel zeroes the running totals
   // A programmatic launch is resident before the one before it has ended, and
   // waits for that first; the kernels of one slot a thread also let the next
   // in at their start.  The capsules' launch is plain: its CTAs and those of
@@ -946,8 +932,7 @@ cudaError_t launch_contact(const ContactArgs& a, cudaStream_t stream, int64_t* l
   };
   go(capsule_kernel, gs, kThreads, false);
   go(cell_kernel, gs, kThreads, true);
-  go(range_kernel, static_cast<unsigned>((table + kThreads * kRangeItems - 1) / (kThreads * kRangeItems)), kThreads,
-     true);
+  go(range_kernel, gs, kThreads, true);
   go(scatter_kernel, gs, kThreads, true);
   const unsigned ge = static_cast<unsigned>((a.n_caps + kThreads - 1) / kThreads);
   int dev = 0, sms = 148;

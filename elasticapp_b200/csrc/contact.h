@@ -86,8 +86,7 @@ struct ContactArgs {
   uint32_t table_mask;               // hash table size - 1 (power of two)
   uint32_t max_cells;                // buckets of the tables below: cells a dense grid may have (at least
                                      // the hash table's size)
-  int32_t* bucket_count;             // max_cells (zero between steps)
-  int2* bucket_range;                // max_cells: a bucket's first entry and the one past its last
+  int2* cell;                        // max_cells: the capsules filed in a bucket and the first one's entry
   ContactGrid* grid;
   ContactRecord* sorted_rec;         // n_caps: the capsules grouped by bucket
   int32_t* pair_count;               // stride (zero outside capsules): partners per capsule (between

@@ -131,8 +131,7 @@ struct ContactDevice {
   int32_t* cap_material = nullptr;
   unsigned long long* extent = nullptr;
   uint32_t* bucket = nullptr;
-  int32_t* bucket_count = nullptr;
-  int2* bucket_range = nullptr;
+  int2* cell = nullptr;
   eb::ContactGrid* grid = nullptr;
   uint8_t* plain_joint = nullptr;
   int32_t* live = nullptr;
@@ -461,7 +460,7 @@ void host_free(eb_sim* s) {
       g = nullptr;
     }
   ContactDevice& c = s->contact;
-  void* cptrs[] = {c.cap, c.cap_material, c.extent, c.bucket, c.bucket_count, c.bucket_range,
+  void* cptrs[] = {c.cap, c.cap_material, c.extent, c.bucket, c.cell,
                    c.grid, c.plain_joint, c.live,
                    c.sorted_rec, c.pair_count, c.fixed, c.pair_offset,
                    c.partners,
@@ -593,8 +592,7 @@ eb_status setup_contact(eb_sim* s) {
   alloc(&c.cap_material, static_cast<size_t>(S) * sizeof(int32_t));
   alloc(&c.extent, sizeof(unsigned long long));
   alloc(&c.bucket, static_cast<size_t>(S) * sizeof(uint32_t));
-  alloc(&c.bucket_count, static_cast<size_t>(c.max_cells) * sizeof(int32_t));
-  alloc(&c.bucket_range, static_cast<size_t>(c.max_cells) * sizeof(int2));
+  alloc(&c.cell, static_cast<size_t>(c.max_cells) * sizeof(int2));
   alloc(&c.grid, sizeof(eb::ContactGrid));
   alloc(&c.plain_joint, static_cast<size_t>(S));
   alloc(&c.live, static_cast<size_t>(n_caps) * sizeof(int32_t));
@@ -1754,8 +1752,7 @@ eb::ContactArgs contact_args(eb_sim* s, double dt) {
   a.bucket = c.bucket;
   a.table_mask = c.table_mask;
   a.max_cells = c.max_cells;
-  a.bucket_count = c.bucket_count;
-  a.bucket_range = c.bucket_range;
+  a.cell = c.cell;
   a.grid = c.grid;
   a.plain_joint = c.plain_joint;
   a.live = c.live;
