@@ -79,9 +79,12 @@ __device__ __forceinline__ Length length_of(double l2) {
   return {l, 1.0 / l};
 }
 
-// The coefficients of so3_update_fast: the rotation is applied to a slot's
-// directors twice a step (the closing half drift of one step and the first of
-// the next have the same angle), so they are formed once.
+// The coefficients of exp(-[u]x): sin(theta) and 1 - cos(theta) from their
+// Taylor series for theta < 0.1 (truncation below 1e-21 relative), which also
+// avoids the cancellation of 1 - cos(theta) at small angles, and one
+// reciprocal for the axis.  The rotation is applied to a slot's directors
+// twice a step (the closing half drift of one step and the first of the next
+// have the same angle), so they are formed once.
 struct Rotation {
   double c, s;      // cos, sin of the angle
   double u[3];      // guarded axis
@@ -117,8 +120,8 @@ __device__ __forceinline__ Rotation rotation(double u0, double u1, double u2) {
   return {1.0 - alpha, s, {u0, u1, u2}, {alpha * u0, alpha * u1, alpha * u2}};
 }
 
-// Q <- R Q; the products are fused as the compiler fuses so3_update_fast
-// (written out, so that every kernel rounds alike)
+// Q <- R Q; which products are fused is written out, so that every kernel
+// rounds alike
 __device__ __forceinline__ void rotate(double q[9], const Rotation& R) {
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
@@ -130,9 +133,10 @@ __device__ __forceinline__ void rotate(double q[9], const Rotation& R) {
   }
 }
 
-// Curvature as inv_rotate_divide_fast forms it, with the square root and the
-// quotient in the forms above (a 1 - cos(theta) outside (1e-12, 2) takes the
-// plain operations).
+// Curvature (inv_rotate_divide in rod_math.cuh) with sin(acos(c) + d) =
+// sqrt((1 - c)(1 + c)) cos d + c sin d, d = 1e-14 (cos d rounds to 1, sin d to
+// d), and the square root and the quotient in the forms above (a 1 - cos(theta)
+// outside (1e-12, 2) takes the plain operations).
 __device__ __forceinline__ Vec3<double> curvature(const double qc[9], const double qn[9], double span) {
   const double tr = qc[0] * qn[0] + qc[1] * qn[1] + qc[2] * qn[2] + qc[3] * qn[3] + qc[4] * qn[4] +
                     qc[5] * qn[5] + qc[6] * qn[6] + qc[7] * qn[7] + qc[8] * qn[8];
