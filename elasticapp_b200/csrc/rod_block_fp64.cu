@@ -22,8 +22,9 @@
 // memory as well (distributed shared memory), so every read is local, and the
 // barriers that order a phase's writes before the next phase's neighbour
 // reads become cluster barriers.  (Reads that go to the partner past the
-// split cost every slot a test and an address, and registers spilled.)  Serving launches mix pairs and single CTAs in one cluster
-// launch; a single CTA takes only CTA barriers.
+// split cost every slot a test and an address, and registers spilled.)  Serving
+// launches mix pairs and single CTAs in one cluster launch; a single CTA takes
+// only CTA barriers.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 

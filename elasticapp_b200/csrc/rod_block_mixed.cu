@@ -19,9 +19,9 @@
 // FP64 values changed, cost 12 shared-memory stores and 12 loads a slot and
 // step for the same values and 48 B of shared memory a slot), and the
 // divisions of the element math are reciprocal square roots and rounded
-// reciprocals (the reciprocals of the masses and Voronoi rest lengths are
-// formed each step rather than stored: shared memory per slot, not the
-// arithmetic, sets how many slots an SM holds).
+// reciprocals (those of the rest lengths stored in entries of float4 rows
+// that were spare; the mass's formed each step: shared memory per slot, not
+// the arithmetic, sets how many slots an SM holds).
 //
 // Reformulations (mathematically identical; rounding differs):
 //   sigma = (Q t) e - z  =  Q dx / l0 - z         (no normalisation)
