@@ -65,6 +65,9 @@ struct ContactGrid {
   unsigned long long scanned;  // records the evaluation before read in its search
   int32_t filed;               // capsules filed in the grid
   int32_t live;                // capsules in the list of those the narrow phase evaluates
+  // entries and listed capsules that the search's and the narrow phase's
+  // warps have taken beyond their first
+  uint32_t searched, evaluated;
   // bounds of the boxes' lower corners, rounded outward to FP32: the largest
   // and the negated smallest as order-preserving integers (zero: none yet)
   uint32_t top[3], bottom[3];
