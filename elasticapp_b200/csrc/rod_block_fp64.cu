@@ -283,13 +283,13 @@ __global__ void __launch_bounds__(kThreads, block_min_ctas<kCap>()) rod_block_fp
       const D3 d = sigma - R.get3(bSig0, s);
       const D3 sh = R.get3(bShear, s);
       const D3 nl = {sh.x * d.x, sh.y * d.y, sh.z * d.z};
-      const double ie = rcp_from(e, l0 * il);
+      const double ie = rcp_from_rough(e, l0 * il);
       o.f = scale(mattranspvec(m.q, nl), ie);
       const D3 J = R.get3(bJ, s);
       const D3 jwe = {J.x * m.w.x * ie, J.y * m.w.y * ie, J.z * m.w.z * ie};
       const D3 dv = R.get3(bV, s + 1) - m.v;
       const double el0 = e * l0;
-      const double rate = div_from(dot(t, dv), el0, rcp_from(el0, il));
+      const double rate = div_from(dot(t, dv), el0, rcp_from_rough(el0, il));
       o.tl = scale(cross(qt, nl), l0) + cross(jwe, m.w) + scale(jwe, rate);
       o.e = e;
       if (meta & kVor) {

@@ -11,9 +11,21 @@
 // (error e -> O(e^3), below an ulp) and a correction by the exact residual
 // (Markstein's theorem), without branches, so that independent chains
 // interleave.
+//
+// What a correction leaves out, the residual's square, is below 2^-100 of the
+// result, so only a reciprocal or root that near to a tie could round wrongly.
+// Those can be listed: with 53-bit significands D and midpoints M / 2^54,
+// 1 / D is near one where D M = 2^106 - k for a small k (126 significands for
+// |k| <= 20, by factoring), a root where M^2 is as near to a multiple of a power
+// of two (only three squares are near enough to matter), a quotient where D M
+// is.  Every such reciprocal and root, and ten thousand such quotients, are
+// compared with the exact result (tests/test_gpu_rod_fast.py).  Of a quotient
+// -0 the sign is lost.
 #pragma once
 
 #include <cuda_runtime.h>
+
+#include <cstdint>
 
 #include "rod_math.cuh"
 
@@ -28,14 +40,22 @@ __device__ __forceinline__ double rcp_near(double d) {
   return fma(y, fma(e, e, e), y);
 }
 
-// 1 / d from an approximation y of it within a few ulps.  The correction
-// multiplies the residual by y or the number after it: for a d just below a
-// power of two (a dilatation of 1 - 2^-53, say) the corrected value is within
-// 2^-105 of a tie, which the larger factor breaks to the right side; for any
-// other d the two round alike.
+// 1 / d from an approximation y of it that is off by little more than its own
+// rounding (half an ulp; rcp_near's is).  The residual r = 1 - d y gives
+// y + y r, short of 1 / d by its square, which matters only where a tie lies
+// between the two: where r > 0, y with its last bit set in y's place makes up
+// for it (where r < 0 no such tie is passed).
 __device__ __forceinline__ double rcp_from(double d, double y) {
-  return fma(fma(-d, y, 1.0), __longlong_as_double(__double_as_longlong(y) | 1ll), y);
+  const double r = fma(-d, y, 1.0);
+  const uint32_t up = ~static_cast<uint32_t>(__double2hiint(r)) >> 31;
+  return fma(r, __hiloint2double(__double2hiint(y), static_cast<int>(static_cast<uint32_t>(__double2loint(y)) | up)), y);
 }
+
+// 1 / d from an approximation y of it within 16 ulps.  (From a start of up to
+// three ulps, one step alone rounds dozens of significands wrongly.  The second
+// takes 2000 steps of a 100-element rod 3.77 -> 3.86 ms, 128 steps of 8192 rods
+// 13.04 -> 13.01.)
+__device__ __forceinline__ double rcp_from_rough(double d, double y) { return rcp_from(d, fma(fma(-d, y, 1.0), y, y)); }
 
 // a / d from y, the rounded 1 / d
 __device__ __forceinline__ double div_from(double a, double d, double y) {
@@ -73,7 +93,10 @@ __device__ __forceinline__ Length length_of(double l2) {
   if (ordinary(l2)) {
     const double y = rsqrt_near(l2);
     const double l = sqrt_from(l2, y);
-    return {l, rcp_from(l, y)};
+    // (y is within 2 ulps of 1 / l: the double after it where the residual is
+    // positive, and the one before it where it is negative, round every one)
+    const double r = fma(-l, y, 1.0);
+    return {l, fma(r, __longlong_as_double(__double_as_longlong(y) + (1 | (__double2hiint(r) >> 31))), y)};
   }
   const double l = sqrt(l2);
   return {l, 1.0 / l};

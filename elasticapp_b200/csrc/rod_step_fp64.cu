@@ -274,7 +274,7 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
       l = len.l;
       const double il = len.il;
       e = div_from(l, l0, rcp_from(l0, rcp_near(l0)));
-      const double ie = rcp_from(e, l0 * il);
+      const double ie = rcp_from_rough(e, l0 * il);
       t = scale(dx, il);
 #else
       l = sqrt(dx.x * dx.x + dx.y * dx.y + dx.z * dx.z);
