@@ -76,12 +76,8 @@ __device__ __forceinline__ void st3(double* p, int64_t S, int64_t s, D3 a) {
 }
 __device__ __forceinline__ D3 mul3(double k, D3 a) { return {k * a.x, k * a.y, k * a.z}; }
 __device__ __forceinline__ D3 neg3(D3 a) { return {-a.x, -a.y, -a.z}; }
-// a / b, 1 / b and sqrt(a) in the correctly rounded forms of rod_fast.cuh
-// (their fused operations are written out, so nothing is contracted here)
-__device__ __forceinline__ double reciprocal(double b) { return ordinary(b) ? rcp_from(b, rcp_near(b)) : 1.0 / b; }
-__device__ __forceinline__ double quotient(double a, double b) {
-  return ordinary(b) ? div_from(a, b, rcp_from(b, rcp_near(b))) : a / b;
-}
+// quotients and roots in the correctly rounded forms of rod_fast.cuh (their
+// fused operations are written out, so nothing is contracted here)
 __device__ __forceinline__ D3 quotient3(D3 a, double b) {
   if (!ordinary(b)) return {a.x / b, a.y / b, a.z / b};
   const double y = rcp_from(b, rcp_near(b));

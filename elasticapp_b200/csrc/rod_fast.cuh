@@ -85,6 +85,20 @@ __device__ __forceinline__ bool ordinary(double d) {
   return static_cast<uint32_t>(__double2hiint(d)) - (623u << 20) < (800u << 20);
 }
 
+// 1 / d and a / d for any d
+__device__ __forceinline__ double reciprocal(double d) { return ordinary(d) ? rcp_from(d, rcp_near(d)) : 1.0 / d; }
+__device__ __forceinline__ double quotient(double a, double d) {
+  return ordinary(d) ? div_from(a, d, rcp_from(d, rcp_near(d))) : a / d;
+}
+
+// The rod kernels take the rest lengths, dilatations and Voronoi lengths
+// without the test.  Outside the range these are those of a rod that has
+// collapsed, blown up or was given no usable length, whose state is no longer
+// finite either way: it turns NaN at once instead of by way of an infinity.
+// (The tests took the resident kernel 4 to 11 % longer: a 100-element rod 3.86
+// -> 4.24 ms, 8192 rods 13.0 -> 13.6.)  Masses are tested: an infinite one
+// holds its node.
+
 // length and reciprocal length from the squared length
 struct Length {
   double l, il;

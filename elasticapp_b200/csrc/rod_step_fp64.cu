@@ -373,7 +373,7 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
     Fe = {Fe.x + jf[g], Fe.y + jf[S + g], Fe.z + jf[2 * S + g]};
   }
 #ifdef EB_FAST_FP64
-  const double inv_m = rcp_from(m, rcp_near(m));
+  const double inv_m = reciprocal(m);
 #else
   const double inv_m = 1.0 / m;
 #endif
