@@ -181,13 +181,17 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
     // Consecutive capsules of a rod share a node, so the narrow phase finds
     // them no distance apart and no contact.  Its tolerance on the projections
     // (1e-8 m^2) can only pick another region for elements shorter than a
-    // millimetre or folded back on one another, and the ends only part by
-    // rounding (1e-8 m) far from the origin: such joints are evaluated.
+    // millimetre or folded back on one another, or where the ends part by so
+    // much rounding that it passes the tolerance: they part by up to
+    // 1.2e-15 (X + 2 L), L the longer element's length and X the coordinates,
+    // and the projections by L times that, 3.5e-9 m^2 within the bound below
+    // (and the ends by 1.2e-9 m, of 1e-8).  Other joints are evaluated.
     {
       const D3 dn = x2 - x1;
-      const double l2 = dot(dx, dx), n2 = dot(dn, dn), along = dot(dx, dn);
-      a.plain_joint[s] = joint && l2 > 1e-6 && n2 > 1e-6 && l2 < 1e8 && n2 < 1e8 && along > 0.0 &&
-                         along * along > 0.01 * (l2 * n2) && fabs(x1.x) < 1e6 && fabs(x1.y) < 1e6 && fabs(x1.z) < 1e6;
+      const double l2 = dot(dx, dx), n2 = dot(dn, dn), along = dot(dx, dn), big = fmax(l2, n2);
+      const double far = fmax(fabs(x1.x), fmax(fabs(x1.y), fabs(x1.z)));
+      a.plain_joint[s] = joint && l2 > 1e-6 && n2 > 1e-6 && far < 1e6 && (far * far + big) * big < 1e12 &&
+                         along > 0.0 && along * along > 0.01 * (l2 * n2);
     }
     D3 t;
     double area;  // volume / (pi l)
