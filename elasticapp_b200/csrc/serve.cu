@@ -365,21 +365,33 @@ eb_status upload_alloc(eb_server* s, size_t bytes, size_t* off) {
   return EB_OK;
 }
 
-// Staging space for `bytes`, copied (by stage_copy) to the same place of the
-// device's copy of the ring; close_stage records when it may be reused (on
-// every path, so the ring's allocations and the events stay paired).
-eb_status close_stage(eb_server* s) {
-  cudaEvent_t ev = nullptr;
-  if (!s->spare_events.empty()) {
-    ev = s->spare_events.back();
-    s->spare_events.pop_back();
-  } else {
-    SV_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+// Staging space for `bytes`, and the same place of the device's copy of the
+// ring.  It may be reused once the event recorded when the stage closes has
+// passed; the event joins the list with the allocation, so that the two stay
+// paired on every path.
+struct Stage {
+  eb_server* s;
+  unsigned char *host = nullptr, *dev = nullptr;
+  explicit Stage(eb_server* server) : s(server) {}
+  ~Stage() {
+    if (host) cudaEventRecord(s->upload_events.back(), s->stream);
   }
-  s->upload_events.push_back(ev);
-  SV_CUDA(cudaEventRecord(ev, s->stream));
-  return EB_OK;
-}
+  eb_status open(size_t bytes) {
+    if (s->spare_events.empty()) {
+      cudaEvent_t fresh = nullptr;
+      SV_CUDA(cudaEventCreateWithFlags(&fresh, cudaEventDisableTiming));
+      s->spare_events.push_back(fresh);
+    }
+    size_t off = 0;
+    if (eb_status st = upload_alloc(s, bytes, &off)) return st;
+    const cudaEvent_t ev = s->spare_events.back();
+    s->spare_events.pop_back();
+    s->upload_events.push_back(ev);
+    host = s->upload.base + off;
+    dev = s->d_upload + off;
+    return EB_OK;
+  }
+};
 
 eb::RodRef rod_ref(const Request& r, size_t k) {
   eb::RodRef ref{};
@@ -391,80 +403,111 @@ eb::RodRef rod_ref(const Request& r, size_t k) {
 
 size_t spec_bytes(size_t rods) { return (rods * (sizeof(eb::RodSpec) + sizeof(eb::RodRef)) + 255) / 256 * 256; }
 
-// Write the initial rods of the requests admitted together into their bins:
-// the rods' specifications and velocities go through pinned staging (so the
-// copy queues behind the running ticks instead of waiting for them), a kernel
-// computes the slots' data there, and another the initial energies.
-eb_status place(eb_server* s, const std::vector<Request*>& batch) {
-  size_t nr = 0, nv = 0;
-  for (const Request* r : batch) {
-    nr += r->rods.size();
-    nv += r->velocities.size();
-  }
-  if (nr == 0) return EB_OK;
+// one rod of a request and its velocities (null: none)
+struct RodAt {
+  Request* r;
+  size_t k;
+  const double* velocities;
+};
+
+// Write the initial data of `nr` rods into their bins: the rods'
+// specifications and velocities go through pinned staging (so the copy queues
+// behind the running ticks instead of waiting for them), a kernel computes the
+// slots' data there, and another the initial energies.
+eb_status place_rods(eb_server* s, const RodAt* rods, size_t nr, size_t nv) {
+  Stage stage(s);
   const size_t uvel = spec_bytes(nr), bytes = uvel + nv * sizeof(double);
-  size_t base_off = 0;
-  if (eb_status st = upload_alloc(s, bytes, &base_off)) return st;
-  unsigned char* base = s->upload.base + base_off;
-  eb::RodSpec* specs = reinterpret_cast<eb::RodSpec*>(base);
+  if (eb_status st = stage.open(bytes)) return st;
+  eb::RodSpec* specs = reinterpret_cast<eb::RodSpec*>(stage.host);
   eb::RodRef* refs = reinterpret_cast<eb::RodRef*>(specs + nr);
-  size_t voff = 0, at = 0;
-  for (Request* r : batch) {
-    const size_t v0 = voff;
-    for (size_t k = 0; k < r->rods.size(); ++k, ++at) {
-      eb::RodSpec spec{};
-      if (eb_status e = eb::straight_rod_spec(r->rods[k], spec)) {
-        close_stage(s);
-        return e;
-      }
-      const int64_t first = r->bins[r->rod_bin[k]] * kBin + r->rod_off[k];
-      spec.start = first;
-      spec.rod = static_cast<uint32_t>(r->rod0 + static_cast<int64_t>(k));
-      spec.velocity = -1;
-      if (!r->velocities.empty()) {
-        spec.velocity = static_cast<int64_t>(voff);
-        voff += static_cast<size_t>(3 * (spec.n + 1));
-      }
-      eb::RodInfo& ri = spec.info;
-      for (int d = 0; d < 3; ++d) ri.clamp_x[d] = spec.origin[d] + 0.0 * spec.step[d];
-      for (int q = 0; q < 9; ++q) ri.clamp_Q[q] = spec.rows[q];
-      ri.damper_t = 1.0;
-      ri.clamp_slot[0] = ri.clamp_slot[1] = -1;
-      ri.torque_slot = -1;
-      if (r->options & EB_REQUEST_CLAMP) {
-        ri.flags |= eb::kRodClamp;
-        ri.clamp_slot[0] = first;  // node 0 / element 0 of the rod
-      }
-      if (r->options & EB_REQUEST_DAMPER) {
-        ri.flags |= eb::kRodDamper;
-        ri.damper_t = std::exp(-r->nu_t * r->dt);
-        ri.damper_r = r->nu_r;
-      }
-      if (spec.damped) r->damped = true;
-      specs[at] = spec;
-      refs[at] = rod_ref(*r, k);
+  double* vel = reinterpret_cast<double*>(stage.host + uvel);
+  size_t voff = 0;
+  for (size_t i = 0; i < nr; ++i) {
+    Request& r = *rods[i].r;
+    const size_t k = rods[i].k;
+    eb::RodSpec spec{};
+    if (eb_status e = eb::straight_rod_spec(r.rods[k], spec)) return e;
+    const int64_t first = r.bins[r.rod_bin[k]] * kBin + r.rod_off[k];
+    spec.start = first;
+    spec.rod = static_cast<uint32_t>(r.rod0 + static_cast<int64_t>(k));
+    spec.velocity = -1;
+    if (rods[i].velocities) {
+      const size_t n = static_cast<size_t>(3 * (spec.n + 1));
+      std::memcpy(vel + voff, rods[i].velocities, n * sizeof(double));
+      spec.velocity = static_cast<int64_t>(voff);
+      voff += n;
     }
-    if (voff > v0)
-      std::memcpy(base + uvel + v0 * sizeof(double), r->velocities.data(), (voff - v0) * sizeof(double));
+    eb::RodInfo& ri = spec.info;
+    for (int d = 0; d < 3; ++d) ri.clamp_x[d] = spec.origin[d] + 0.0 * spec.step[d];
+    for (int q = 0; q < 9; ++q) ri.clamp_Q[q] = spec.rows[q];
+    ri.damper_t = 1.0;
+    ri.clamp_slot[0] = ri.clamp_slot[1] = -1;
+    ri.torque_slot = -1;
+    if (r.options & EB_REQUEST_CLAMP) {
+      ri.flags |= eb::kRodClamp;
+      ri.clamp_slot[0] = first;  // node 0 / element 0 of the rod
+    }
+    if (r.options & EB_REQUEST_DAMPER) {
+      ri.flags |= eb::kRodDamper;
+      ri.damper_t = std::exp(-r.nu_t * r.dt);
+      ri.damper_r = r.nu_r;
+    }
+    if (spec.damped) r.damped = true;
+    specs[i] = spec;
+    refs[i] = rod_ref(r, k);
   }
-  unsigned char* dev = s->d_upload + base_off;
-  SV_CUDA(cudaMemcpyAsync(dev, base, bytes, cudaMemcpyHostToDevice, s->stream));
-  const eb::RodSpec* dspecs = reinterpret_cast<const eb::RodSpec*>(dev);
+  SV_CUDA(cudaMemcpyAsync(stage.dev, stage.host, bytes, cudaMemcpyHostToDevice, s->stream));
+  const eb::RodSpec* dspecs = reinterpret_cast<const eb::RodSpec*>(stage.dev);
   const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(dspecs + nr);
-  SV_CUDA(eb::launch_rod_init(dspecs, static_cast<int64_t>(nr), reinterpret_cast<const double*>(dev + uvel), s->stride,
-                              s->state[s->cur], s->par, s->meta, s->rods, s->rod_start, s->rod_n, s->stream));
+  SV_CUDA(eb::launch_rod_init(dspecs, static_cast<int64_t>(nr), reinterpret_cast<const double*>(stage.dev + uvel),
+                              s->stride, s->state[s->cur], s->par, s->meta, s->rods, s->rod_start, s->rod_n,
+                              s->stream));
   SV_CUDA(eb::launch_rod_energy_list(drefs, static_cast<int64_t>(nr), s->stride, s->rod_start, s->rod_n,
                                      s->state[s->cur], s->par, s->e0, s->stream));
-  return close_stage(s);
+  return EB_OK;
+}
+
+// the rods of the requests, as much at a time as half the staging ring holds
+// (however large a request, its initial data pass through the ring in parts)
+eb_status place(eb_server* s, const std::vector<Request*>& batch) {
+  std::vector<RodAt> rods;
+  size_t nv = 0;
+  for (Request* r : batch) {
+    const double* v = r->velocities.empty() ? nullptr : r->velocities.data();
+    for (size_t k = 0; k < r->rods.size(); ++k) {
+      const size_t n = v ? static_cast<size_t>(3 * (r->rods[k].n_elements + 1)) : 0;
+      if (!rods.empty() && spec_bytes(rods.size() + 1) + (nv + n) * sizeof(double) > kUploadBytes / 2) {
+        if (eb_status st = place_rods(s, rods.data(), rods.size(), nv)) return st;
+        rods.clear();
+        nv = 0;
+      }
+      rods.push_back({r, k, v});
+      nv += n;
+      if (v) v += n;
+    }
+  }
+  return rods.empty() ? EB_OK : place_rods(s, rods.data(), rods.size(), nv);
+}
+
+// give a request's bins and rod ids back (what is enqueued on them runs before
+// any later use of them on this stream)
+void give_back(eb_server* s, const Request& r) {
+  for (size_t b = 0; b < r.bins.size(); ++b) {
+    if (r.bin_pair[b])
+      s->bins.give_pair(r.bins[b]);
+    else
+      s->bins.give_single(r.bins[b]);
+  }
+  s->rod_ids.release(r.rod0, static_cast<int64_t>(r.rods.size()));
 }
 
 // Admit what fits, first come first served; the requests admitted in one tick
-// are placed together (as much at a time as half the staging ring holds).
+// are placed together.  They leave the queue once they are placed: on an error
+// they stay in it and their bins are given back.
 eb_status admit(eb_server* s) {
   std::vector<Request*> batch;
-  size_t bytes = 0;
-  while (!s->queue.empty()) {
-    Request& r = *s->queue.front();
+  for (Request* q : s->queue) {
+    Request& r = *q;
     pack(r);
     int64_t n_pairs = 0, n_singles = 0;
     unit_counts(r, &n_pairs, &n_singles);
@@ -479,20 +522,19 @@ eb_status admit(eb_server* s) {
       if (!r.bin_pair[b]) r.bins[b] = s->bins.take_single();
     r.steps_done = 0;
     r.damped = false;
-    const size_t need = spec_bytes(r.rods.size()) + r.velocities.size() * sizeof(double);
-    if (!batch.empty() && bytes + need > kUploadBytes / 2) {
-      if (eb_status e = place(s, batch)) return e;
-      batch.clear();
-      bytes = 0;
-    }
-    batch.push_back(&r);
-    bytes += need;
-    if (r.queued_s < 0.0) r.queued_s = std::chrono::duration<double>(Clock::now() - r.t_submit).count();
-    r.state = kActive;
-    s->queue.pop_front();
-    s->active.push_back(&r);
+    batch.push_back(q);
   }
-  return place(s, batch);
+  if (eb_status st = place(s, batch)) {
+    for (const Request* r : batch) give_back(s, *r);
+    return st;
+  }
+  for (Request* r : batch) {
+    if (r->queued_s < 0.0) r->queued_s = std::chrono::duration<double>(Clock::now() - r->t_submit).count();
+    r->state = kActive;
+    s->queue.pop_front();
+    s->active.push_back(r);
+  }
+  return EB_OK;
 }
 
 eb_status poll_events(eb_server* s, bool block_oldest);
@@ -505,9 +547,9 @@ eb_status retire_batch(eb_server* s, const std::vector<Request*>& batch) {
   for (const Request* r : batch) nr += r->rods.size();
   if (nr == 0) return EB_OK;
   const size_t bytes = nr * sizeof(eb::RodRef);
-  size_t base_off = 0;
-  if (eb_status st = upload_alloc(s, bytes, &base_off)) return st;
-  eb::RodRef* refs = reinterpret_cast<eb::RodRef*>(s->upload.base + base_off);
+  Stage stage(s);
+  if (eb_status st = stage.open(bytes)) return st;
+  eb::RodRef* refs = reinterpret_cast<eb::RodRef*>(stage.host);
   for (Request* r : batch) {
     double* dst = reinterpret_cast<double*>(s->arena.base + r->arena_off);
     int64_t at = 0;
@@ -524,26 +566,16 @@ eb_status retire_batch(eb_server* s, const std::vector<Request*>& batch) {
       *refs++ = ref;
     }
   }
-  unsigned char* dev = s->d_upload + base_off;
-  const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(dev);
-  SV_CUDA(cudaMemcpyAsync(dev, s->upload.base + base_off, bytes, cudaMemcpyHostToDevice, s->stream));
+  const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(stage.dev);
+  SV_CUDA(cudaMemcpyAsync(stage.dev, stage.host, bytes, cudaMemcpyHostToDevice, s->stream));
   SV_CUDA(eb::launch_rod_energy_list(drefs, static_cast<int64_t>(nr), s->stride, s->rod_start, s->rod_n,
                                      s->state[s->cur], s->par, s->e1, s->stream));
   SV_CUDA(eb::launch_rod_result(drefs, static_cast<int64_t>(nr), s->stride, s->state[s->cur], s->rod_start, s->rod_n,
                                 s->e0, s->e1, s->stream));
-  if (eb_status st = close_stage(s)) return st;
   for (Request* r : batch) {
     if (!r->event) SV_CUDA(cudaEventCreateWithFlags(&r->event, cudaEventDisableTiming));
     SV_CUDA(cudaEventRecord(r->event, s->stream));
-    // bins and rod ids go back at once: the launches above run before any
-    // later use of them on this stream
-    for (size_t b = 0; b < r->bins.size(); ++b) {
-      if (r->bin_pair[b])
-        s->bins.give_pair(r->bins[b]);
-      else
-        s->bins.give_single(r->bins[b]);
-    }
-    s->rod_ids.release(r->rod0, static_cast<int64_t>(r->rods.size()));
+    give_back(s, *r);
     r->state = kFinishing;
     s->finishing.push_back(r);
   }
