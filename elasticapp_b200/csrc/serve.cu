@@ -212,6 +212,7 @@ struct Request {
   // completion
   cudaEvent_t event = nullptr;
   size_t arena_off = 0;
+  bool arena_held = false;  // the result has its place in the arena
   double e0 = 0.0, e1 = 0.0, escale = 0.0;
   std::vector<double> result;  // per rod, kStateFields rows of n + 1 slots
   std::vector<int64_t> result_off;
@@ -539,18 +540,29 @@ eb_status admit(eb_server* s) {
 
 eb_status poll_events(eb_server* s, bool block_oldest);
 
-// Enqueue the retirement of requests whose last step ran in this tick, for
-// which the arena has room: their final energies, then their results into the
-// arena, a launch each for all of them.
-eb_status retire_batch(eb_server* s, const std::vector<Request*>& batch) {
-  size_t nr = 0;
-  for (const Request* r : batch) nr += r->rods.size();
-  if (nr == 0) return EB_OK;
-  const size_t bytes = nr * sizeof(eb::RodRef);
+// Enqueue the listed rods' final energies and results, a launch each.
+eb_status result_rods(eb_server* s, const std::vector<eb::RodRef>& rods) {
+  const size_t bytes = rods.size() * sizeof(eb::RodRef);
   Stage stage(s);
   if (eb_status st = stage.open(bytes)) return st;
-  eb::RodRef* refs = reinterpret_cast<eb::RodRef*>(stage.host);
+  std::memcpy(stage.host, rods.data(), bytes);
+  const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(stage.dev);
+  SV_CUDA(cudaMemcpyAsync(stage.dev, stage.host, bytes, cudaMemcpyHostToDevice, s->stream));
+  SV_CUDA(eb::launch_rod_energy_list(drefs, static_cast<int64_t>(rods.size()), s->stride, s->rod_start, s->rod_n,
+                                     s->state[s->cur], s->par, s->e1, s->stream));
+  SV_CUDA(eb::launch_rod_result(drefs, static_cast<int64_t>(rods.size()), s->stride, s->state[s->cur], s->rod_start,
+                                s->rod_n, s->e0, s->e1, s->stream));
+  return EB_OK;
+}
+
+// Enqueue the retirement of finished requests, which hold their place in the
+// arena: as many rods at a time as half the staging ring holds.  On an error
+// they stay active.
+eb_status retire_batch(eb_server* s, std::vector<Request*>& batch) {
+  if (batch.empty()) return EB_OK;
+  std::vector<eb::RodRef> refs;
   for (Request* r : batch) {
+    if (!r->event) SV_CUDA(cudaEventCreateWithFlags(&r->event, cudaEventDisableTiming));
     double* dst = reinterpret_cast<double*>(s->arena.base + r->arena_off);
     int64_t at = 0;
     r->result_off.assign(r->rods.size(), 0);
@@ -563,53 +575,64 @@ eb_status retire_batch(eb_server* s, const std::vector<Request*>& batch) {
       ref.result = dst + r->result_off[k];
       ref.energies = dst + at + 5 * k;
       ref.final_at = 5 * static_cast<int64_t>(r->rods.size());
-      *refs++ = ref;
+      refs.push_back(ref);
+      if ((refs.size() + 1) * sizeof(eb::RodRef) > kUploadBytes / 2) {
+        if (eb_status st = result_rods(s, refs)) return st;
+        refs.clear();
+      }
     }
   }
-  const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(stage.dev);
-  SV_CUDA(cudaMemcpyAsync(stage.dev, stage.host, bytes, cudaMemcpyHostToDevice, s->stream));
-  SV_CUDA(eb::launch_rod_energy_list(drefs, static_cast<int64_t>(nr), s->stride, s->rod_start, s->rod_n,
-                                     s->state[s->cur], s->par, s->e1, s->stream));
-  SV_CUDA(eb::launch_rod_result(drefs, static_cast<int64_t>(nr), s->stride, s->state[s->cur], s->rod_start, s->rod_n,
-                                s->e0, s->e1, s->stream));
+  if (!refs.empty())
+    if (eb_status st = result_rods(s, refs)) return st;
   for (Request* r : batch) {
-    if (!r->event) SV_CUDA(cudaEventCreateWithFlags(&r->event, cudaEventDisableTiming));
     SV_CUDA(cudaEventRecord(r->event, s->stream));
     give_back(s, *r);
     r->state = kFinishing;
     s->finishing.push_back(r);
   }
+  batch.clear();
   return EB_OK;
 }
 
-eb_status retire(eb_server* s, const std::vector<Request*>& done) {
+bool finished(const Request& r) { return r.steps_done >= r.n_steps; }
+
+size_t result_bytes(const Request& r) {
+  size_t slots = 0;
+  for (int32_t c : r.bin_count) slots += static_cast<size_t>(c);
+  return (slots * eb::kStateFields + 10 * r.rods.size()) * sizeof(double);
+}
+
+// Retire the active requests whose last step has run.  One whose result the
+// arena can never hold stays active, with its bins, and is reported by every
+// tick (undeliverable).
+eb_status retire(eb_server* s) {
   std::vector<Request*> batch;
-  size_t refs = 0;
-  for (Request* r : done) {
-    const size_t nr = r->rods.size();
-    size_t slots = 0;
-    for (int32_t c : r->bin_count) slots += static_cast<size_t>(c);
-    const size_t bytes = (slots * eb::kStateFields + 10 * nr) * sizeof(double);
-    if (!batch.empty() && (refs + nr) * sizeof(eb::RodRef) > kUploadBytes / 2) {
-      if (eb_status st = retire_batch(s, batch)) return st;
-      batch.clear();
-      refs = 0;
-    }
-    while (!s->arena.alloc(bytes, &r->arena_off)) {
+  eb_status st = EB_OK;
+  for (Request* r : s->active) {
+    if (!finished(*r) || result_bytes(*r) > s->arena.cap) continue;
+    while (st == EB_OK && !r->arena_held) {
+      r->arena_held = s->arena.alloc(result_bytes(*r), &r->arena_off);
+      if (r->arena_held) break;
       // the arena is full: enqueue what has its room, then wait for the
       // oldest retirement and take it out
-      if (!batch.empty()) {
-        if (eb_status st = retire_batch(s, batch)) return st;
-        batch.clear();
-        refs = 0;
-      }
-      if (s->finishing.empty()) return fail(EB_ERR_OUT_OF_MEMORY, "request result larger than the host arena");
-      if (eb_status st = poll_events(s, true)) return st;
+      st = retire_batch(s, batch);
+      if (st == EB_OK && s->finishing.empty()) st = fail(EB_ERR_OUT_OF_MEMORY, "the host arena is in use");
+      if (st == EB_OK) st = poll_events(s, true);
     }
+    if (st != EB_OK) break;
     batch.push_back(r);
-    refs += nr;
   }
-  return retire_batch(s, batch);
+  if (st == EB_OK) st = retire_batch(s, batch);
+  s->active.erase(std::remove_if(s->active.begin(), s->active.end(), [](const Request* r) { return r->state != kActive; }),
+                  s->active.end());
+  return st;
+}
+
+eb_status undeliverable(const eb_server* s) {
+  for (const Request* r : s->active)
+    if (finished(*r) && result_bytes(*r) > s->arena.cap)
+      return fail(EB_ERR_OUT_OF_MEMORY, "request result larger than the host arena");
+  return EB_OK;
 }
 
 // Take a landed retirement out of the arena: energies, drift check, result.
@@ -642,6 +665,7 @@ void land(eb_server* s, Request& r) {
   r.escale = scale;
   r.result.assign(src, src + slots * eb::kStateFields);  // per rod, at its result_off
   s->arena.free_oldest();
+  r.arena_held = false;
   const bool drift_ok = finite && (E1 - E0) <= s->cfg.energy_tolerance * (scale > 0.0 ? scale : 1.0) &&
                        !(s->cfg.flags & EB_SERVER_FORCE_FALLBACK);
   if (!drift_ok && r.precision == EB_PRECISION_MIXED) {
@@ -838,6 +862,8 @@ EB_API eb_status eb_server_tick(eb_server* s, int64_t* in_flight) {
     }
   }
   if (eb_status st = poll_events(s, false)) return st;
+  // what an error kept from retiring, while its final state is the current one
+  if (eb_status st = retire(s)) return st;
   if (eb_status st = admit(s)) return st;
   const int K = s->cfg.steps_per_launch;
   int n_cta[2] = {0, 0};
@@ -848,6 +874,7 @@ EB_API eb_status eb_server_tick(eb_server* s, int64_t* in_flight) {
     for (Request* r : s->active) {
       const int p = r->precision == EB_PRECISION_MIXED ? 0 : 1;
       const int32_t steps = static_cast<int32_t>(std::min<int64_t>(K, r->n_steps - r->steps_done));
+      if (steps == 0) continue;
       for (size_t b = 0; b < r->bins.size(); ++b) {
         if ((pass == 0) != (r->bin_pair[b] != 0)) continue;
         const int halves = r->bin_pair[b] ? 2 : 1;
@@ -896,22 +923,20 @@ EB_API eb_status eb_server_tick(eb_server* s, int64_t* in_flight) {
     }
     if (s->launch_timed[parity]) SV_CUDA(cudaEventRecord(s->launch_t1[parity], s->stream));
     s->cur ^= 1;
-    std::vector<Request*> still, done;
     for (Request* r : s->active) {
       const int64_t steps = std::min<int64_t>(K, r->n_steps - r->steps_done);
       r->steps_done += steps;
       s->element_steps += static_cast<double>(steps) * static_cast<double>(r->elements);
-      (r->steps_done >= r->n_steps ? done : still).push_back(r);
     }
-    s->active.swap(still);
-    if (eb_status st = retire(s, done)) return st;
   }
+  // (before the retirement, which may fail: the launches use the tables)
   SV_CUDA(cudaEventRecord(s->tick_event[parity], s->stream));
   s->tick_pending[parity] = true;
   ++s->ticks;
+  if (eb_status st = retire(s)) return st;
   if (in_flight)
     *in_flight = static_cast<int64_t>(s->queue.size() + s->active.size() + s->finishing.size());
-  return EB_OK;
+  return undeliverable(s);
 }
 
 EB_API eb_status eb_server_poll(eb_server* s, eb_completion* out, int32_t capacity, int32_t* count) {
