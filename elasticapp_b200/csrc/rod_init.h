@@ -1,5 +1,5 @@
 // Initial data of straight rods on the device, and their final state to the
-// host (rod_init.cu).
+// host (rod_init.cu).  The lists and velocities may be pinned host memory.
 #pragma once
 
 #include <cuda_runtime.h>

@@ -244,10 +244,9 @@ struct eb_server {
   int cur = 0;
   int64_t ticks = 0;
   Ring arena;
-  // pinned staging of initial data: copies from pageable memory would wait
-  // for the stream (the running ticks) before each admission
+  // pinned staging of initial data and lists of results: copies from pageable
+  // memory would wait for the stream (the running ticks) before each admission
   Ring upload;
-  unsigned char* d_upload = nullptr;  // the device's copy of it
   std::deque<cudaEvent_t> upload_events;  // one per live upload allocation, in order
   std::vector<cudaEvent_t> spare_events;
   BinPool bins;
@@ -267,7 +266,7 @@ namespace {
 void server_free(eb_server* s) {
   cudaSetDevice(s->cfg.device);
   if (s->stream) cudaStreamSynchronize(s->stream);
-  void* dev[] = {s->state[0], s->state[1], s->par, s->meta, s->rods, s->rod_start, s->rod_n, s->e0, s->e1, s->status, s->d_upload};
+  void* dev[] = {s->state[0], s->state[1], s->par, s->meta, s->rods, s->rod_start, s->rod_n, s->e0, s->e1, s->status};
   for (void* p : dev)
     if (p) cudaFree(p);
   for (int a = 0; a < 2; ++a)
@@ -366,13 +365,14 @@ eb_status upload_alloc(eb_server* s, size_t bytes, size_t* off) {
   return EB_OK;
 }
 
-// Staging space for `bytes`, and the same place of the device's copy of the
-// ring.  It may be reused once the event recorded when the stage closes has
-// passed; the event joins the list with the allocation, so that the two stay
-// paired on every path.
+// Staging space for `bytes`, read by the kernels where it lies: a copy of the
+// ring on the device would take 128 MiB beside the pool that the server's
+// budget pays for.  It may be reused once the event recorded when the stage
+// closes has passed; the event joins the list with the allocation, so that the
+// two stay paired on every path.
 struct Stage {
   eb_server* s;
-  unsigned char *host = nullptr, *dev = nullptr;
+  unsigned char* host = nullptr;
   explicit Stage(eb_server* server) : s(server) {}
   ~Stage() {
     if (host) cudaEventRecord(s->upload_events.back(), s->stream);
@@ -389,7 +389,6 @@ struct Stage {
     s->spare_events.pop_back();
     s->upload_events.push_back(ev);
     host = s->upload.base + off;
-    dev = s->d_upload + off;
     return EB_OK;
   }
 };
@@ -412,9 +411,9 @@ struct RodAt {
 };
 
 // Write the initial data of `nr` rods into their bins: the rods'
-// specifications and velocities go through pinned staging (so the copy queues
-// behind the running ticks instead of waiting for them), a kernel computes the
-// slots' data there, and another the initial energies.
+// specifications and velocities go through pinned staging (nothing waits for
+// the running ticks), from which a kernel computes the slots' data, and another
+// the initial energies.
 eb_status place_rods(eb_server* s, const RodAt* rods, size_t nr, size_t nv) {
   Stage stage(s);
   const size_t uvel = spec_bytes(nr), bytes = uvel + nv * sizeof(double);
@@ -457,13 +456,9 @@ eb_status place_rods(eb_server* s, const RodAt* rods, size_t nr, size_t nv) {
     specs[i] = spec;
     refs[i] = rod_ref(r, k);
   }
-  SV_CUDA(cudaMemcpyAsync(stage.dev, stage.host, bytes, cudaMemcpyHostToDevice, s->stream));
-  const eb::RodSpec* dspecs = reinterpret_cast<const eb::RodSpec*>(stage.dev);
-  const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(dspecs + nr);
-  SV_CUDA(eb::launch_rod_init(dspecs, static_cast<int64_t>(nr), reinterpret_cast<const double*>(stage.dev + uvel),
-                              s->stride, s->state[s->cur], s->par, s->meta, s->rods, s->rod_start, s->rod_n,
-                              s->stream));
-  SV_CUDA(eb::launch_rod_energy_list(drefs, static_cast<int64_t>(nr), s->stride, s->rod_start, s->rod_n,
+  SV_CUDA(eb::launch_rod_init(specs, static_cast<int64_t>(nr), vel, s->stride, s->state[s->cur], s->par, s->meta,
+                              s->rods, s->rod_start, s->rod_n, s->stream));
+  SV_CUDA(eb::launch_rod_energy_list(refs, static_cast<int64_t>(nr), s->stride, s->rod_start, s->rod_n,
                                      s->state[s->cur], s->par, s->e0, s->stream));
   return EB_OK;
 }
@@ -546,11 +541,10 @@ eb_status result_rods(eb_server* s, const std::vector<eb::RodRef>& rods) {
   Stage stage(s);
   if (eb_status st = stage.open(bytes)) return st;
   std::memcpy(stage.host, rods.data(), bytes);
-  const eb::RodRef* drefs = reinterpret_cast<const eb::RodRef*>(stage.dev);
-  SV_CUDA(cudaMemcpyAsync(stage.dev, stage.host, bytes, cudaMemcpyHostToDevice, s->stream));
-  SV_CUDA(eb::launch_rod_energy_list(drefs, static_cast<int64_t>(rods.size()), s->stride, s->rod_start, s->rod_n,
+  const eb::RodRef* refs = reinterpret_cast<const eb::RodRef*>(stage.host);
+  SV_CUDA(eb::launch_rod_energy_list(refs, static_cast<int64_t>(rods.size()), s->stride, s->rod_start, s->rod_n,
                                      s->state[s->cur], s->par, s->e1, s->stream));
-  SV_CUDA(eb::launch_rod_result(drefs, static_cast<int64_t>(rods.size()), s->stride, s->state[s->cur], s->rod_start,
+  SV_CUDA(eb::launch_rod_result(refs, static_cast<int64_t>(rods.size()), s->stride, s->state[s->cur], s->rod_start,
                                 s->rod_n, s->e0, s->e1, s->stream));
   return EB_OK;
 }
@@ -762,7 +756,6 @@ EB_API eb_status eb_server_create(const eb_server_config* config, eb_server** ou
   alloc(&s->e0, static_cast<size_t>(s->rod_cap) * 5 * sizeof(double));
   alloc(&s->e1, static_cast<size_t>(s->rod_cap) * 5 * sizeof(double));
   alloc(&s->status, sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&s->d_upload), kUploadBytes);
   for (int a = 0; a < 2; ++a)
     for (int b = 0; b < 2; ++b) {
       // one entry per bin, plus the padding entry of an odd count

@@ -1,5 +1,6 @@
-"""The server at its limits (GPU): requests whose initial data need several
-stages, results that cannot be delivered or wait for room."""
+"""The server at its limits (GPU): device memory within the budget, requests
+whose initial data need several stages, results that cannot be delivered or
+wait for room."""
 import numpy as np
 import pytest
 
@@ -13,6 +14,18 @@ FIELDS = ("Position", "Velocity", "Director", "AngularVelocity")
 
 def rod(n, k=0):
     return eb.StraightRod(n, eb.Material(1000.0, 1e6, 3e5), 0.01, 1.0, origin=(0.0, 1e-3 * k, 0.0))
+
+
+def test_device_memory_within_the_budget():
+    import torch
+
+    Server(hbm_budget_bytes=2e8).close()  # the context and the module
+    before, _ = torch.cuda.mem_get_info(0)
+    srv = Server(hbm_budget_bytes=2e8)
+    after, _ = torch.cuda.mem_get_info(0)
+    srv.close()
+    # 14 allocations, each rounded up to a granule of 2 MiB
+    assert before - after <= 2e8 + 28 * 2 ** 20
 
 
 def test_admission_in_several_stages():
