@@ -239,6 +239,7 @@ struct eb_sim {
   int64_t xplan = -1;
   cudaStream_t xs[4] = {nullptr, nullptr, nullptr, nullptr};
   std::vector<cudaEvent_t> xev;
+  cudaEvent_t x_inputs = nullptr;  // the inputs of an exchange in sequence have landed
   // captured streaming steps: per starting buffer parity, for graph_dt
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   double graph_dt[2] = {0.0, 0.0};
@@ -692,6 +693,7 @@ EB_API eb_status eb_sim_destroy(eb_sim* s) {
     if (x) cudaStreamSynchronize(x);
   host_free(s);
   for (cudaEvent_t e : s->xev) cudaEventDestroy(e);
+  if (s->x_inputs) cudaEventDestroy(s->x_inputs);
   for (cudaStream_t x : s->xs)
     if (x) cudaStreamDestroy(x);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -2112,9 +2114,10 @@ EB_API eb_status eb_step_host_state(eb_sim* s, double* time, double dt, int64_t 
     overlap = !s->xgroups.empty();
   }
   if (!overlap) {
-    // every copy is queued on the stream, and the host waits once, at the end
-    // (waiting for each field and each status word took 70 of the 279 us that
-    // 32 one-step calls of a 100-element rod and the read of its state take)
+    // every copy is queued on the stream, and the host waits once: for the
+    // outputs, or without any for the inputs (waiting for each field and each
+    // status word took 70 of the 279 us that 32 one-step calls of a 100-element
+    // rod and the read of its state take)
     const size_t w = static_cast<size_t>(s->n_slots) * sizeof(double);
     const size_t dev_pitch = static_cast<size_t>(s->stride) * sizeof(double);
     bool any_in = false;
@@ -2127,6 +2130,10 @@ EB_API eb_status eb_step_host_state(eb_sim* s, double* time, double dt, int64_t 
         EB_CUDA(cudaMemcpy2DAsync(base, dev_pitch, in[f], w, w, fi.ncomp, cudaMemcpyHostToDevice, s->stream));
         EB_CUDA(cudaMemcpy2DAsync(s->d_state[s->cur ^ 1] + fi.offset * s->stride, dev_pitch, base, dev_pitch, w,
                                   fi.ncomp, cudaMemcpyDeviceToDevice, s->stream));
+      }
+      if (any_in && !any_out) {
+        if (!s->x_inputs) EB_CUDA(cudaEventCreateWithFlags(&s->x_inputs, cudaEventDisableTiming));
+        EB_CUDA(cudaEventRecord(s->x_inputs, s->stream));
       }
       if (eb_status st = eb_step(s, time, dt, n_steps)) return st;
       for (int f = 0; f < 4; ++f) {
@@ -2144,7 +2151,7 @@ EB_API eb_status eb_step_host_state(eb_sim* s, double* time, double dt, int64_t 
       return st;
     }
     if (any_out) return check_device_status(s);
-    if (any_in) EB_CUDA(cudaStreamSynchronize(s->stream));
+    if (any_in) EB_CUDA(cudaEventSynchronize(s->x_inputs));
     return EB_OK;
   }
   if (eb_status st = damper_for_dt(s, dt)) return st;
