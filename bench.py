@@ -69,11 +69,25 @@ def source_digest(*names: str) -> str:
     return h.hexdigest()[:16]
 
 
+def with_headers(*names: str) -> list[str]:
+    """The named kernel sources and the headers beside them that they include,
+    directly or through one another, in the order met."""
+    import re
+
+    found = list(names)
+    for n in found:
+        with open(os.path.join(ROOT, "elasticapp_b200", "csrc", n), encoding="utf-8") as f:
+            for h in re.findall(r'^#include "([^"/]+)"', f.read(), re.M):
+                if h not in found:
+                    found.append(h)
+    return found
+
+
 def profile_traffic(kernel: str, workload: str, sources: tuple, elements: int):
     """DRAM bytes per launch from the committed ncu summary of this kernel
     and workload, if its recorded source digest matches the kernel sources
-    as they are now (a summary of an older kernel is not reported) and it
-    covers a launch over the same number of elements.
+    and their headers as they are now (a summary of an older kernel is not
+    reported) and it covers a launch over the same number of elements.
     Returns (bytes or None, note)."""
     path = os.path.join(ROOT, "profiles", f"{kernel}_{workload}.txt")
     traffic, digest, covered = None, None, None
@@ -88,7 +102,7 @@ def profile_traffic(kernel: str, workload: str, sources: tuple, elements: int):
                     covered = int(line.split(":", 1)[1].strip())
     except OSError:
         return None, "no ncu summary"
-    now = source_digest(*sources)
+    now = source_digest(*with_headers(*sources))
     if digest != now:
         return None, f"stale ncu summary ({digest} != {now})"
     if covered != elements:
