@@ -35,8 +35,12 @@ struct P3 {
   double x, y, z;
 };
 
-// joints a slot may carry for its thread to evaluate them itself
-constexpr int kFewJoints = 8;
+// joints a slot may carry for its thread to evaluate them itself.  A joint
+// more is a chain of loads, a root and divisions more in that thread: 64 rods
+// with k others jointed to one node, us a step with one launch and with two,
+// k = 2: 10.3 and 10.7, 4: 13.4 and 11.5, 8: 18.3 and 12.7, 16: 27.9 and 15.0
+// (hinges 10.4 and 11.8, 13.4 and 12.4, 18.4 and 13.4, 27.9 and 16.1)
+constexpr int kFewJoints = 2;
 
 __device__ __forceinline__ P3 node_position(const JointArgs& a, int64_t g) {
   const uint32_t m = a.meta[g];
@@ -142,7 +146,7 @@ __global__ void joint_apply_kernel(const JointArgs a) {
 }  // namespace
 
 // A launch is a few microseconds of latency and more of host time, so where no
-// slot carries more than a few joints one launch evaluates and sums (a joint
+// slot carries more than two joints one launch evaluates and sums (a joint
 // is then evaluated by each slot it acts on), and a launch begins before the
 // one before it has ended, as the step kernel after it does.  A chain of 32
 // links: 17.5 us a step with two plain launches, 10.3 with two of these,
