@@ -1,7 +1,8 @@
-// Cheaper forms of the FP64 rod arithmetic for the resident kernel, each with
-// the result of the plain expression it stands for.
+// Cheaper forms of the FP64 rod arithmetic for the resident and streaming
+// kernels and the contact search, each with the result of the plain expression
+// it stands for.
 //
-// The kernel is bound by FP64 issue and by the latency of dependent FP64
+// The resident kernel is bound by FP64 issue and by the latency of dependent FP64
 // operations, and a library division or square root is ten or more of them
 // with a branch of its own.  Stiff rods amplify any difference in rounding
 // (two correct evaluations part by 1e-9 in the angular velocities within a
@@ -96,8 +97,8 @@ __device__ __forceinline__ double quotient(double a, double d) {
 // collapsed, blown up or was given no usable length, whose state is no longer
 // finite either way: it turns NaN at once instead of by way of an infinity.
 // (The tests took the resident kernel 4 to 11 % longer: a 100-element rod 3.86
-// -> 4.24 ms, 8192 rods 13.0 -> 13.6.)  Masses are tested: an infinite one
-// holds its node.
+// -> 4.24 ms, 8192 rods 13.0 -> 13.6.)  Masses are not left so: an infinite
+// one holds its node.
 
 // length and reciprocal length from the squared length
 struct Length {

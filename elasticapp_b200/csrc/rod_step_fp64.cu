@@ -196,8 +196,11 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
     if (s < kParamFields && M::needed(s))
       bulk_g2s(R.row(M::param(s)) + off, a.par + s * S + lo, bytes, s == kMass ? bar : bar + 1);
   };
-  // (the CTAs that may have to wait; the others need the state first)
-  const bool early = blockIdx.x < 148u * MinBlocks;
+  // (the CTAs that may have to wait, the first to be resident; the others need
+  // the state first.  Only when the copies are issued depends on it, so the
+  // number of SMs is a B200's, not asked for.)
+  constexpr unsigned kSms = 148;
+  const bool early = blockIdx.x < kSms * MinBlocks;
   if (early) copy_parameters();
   grid_dependency_launch();
   grid_dependency_wait();
@@ -373,7 +376,8 @@ __device__ __forceinline__ void rod_step_window(const StepArgs& a, double* smem)
     Fe = {Fe.x + jf[g], Fe.y + jf[S + g], Fe.z + jf[2 * S + g]};
   }
 #ifdef EB_FAST_FP64
-  const double inv_m = reciprocal(m);
+  // (no acceleration for an infinite mass, or one whose reciprocal is not a normal number)
+  const double inv_m = m > 0x1p1022 ? 0.0 : rcp_from(m, rcp_near(m));
 #else
   const double inv_m = 1.0 / m;
 #endif
