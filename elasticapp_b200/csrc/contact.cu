@@ -96,8 +96,8 @@ __device__ __forceinline__ D3 normalize3(D3 a) {
 // a capsule's shape (centre, axis, length, radius); its velocity and
 // angular velocity are read from the table only where a contact point needs
 // them, so they are not held in registers through the closest-point search
-// (that took the narrow phase's spills from 108 to 52 B a thread and the
-// contact step from 0.71 to 0.69 ms)
+// (that took the contact step from 0.71 to 0.69 ms; 68 B a thread of the
+// narrow phase are still spilled)
 struct Capsule {
   D3 c, u;
   double L, r;
@@ -289,8 +289,13 @@ __global__ void __launch_bounds__(kThreads) capsule_kernel(const ContactArgs a) 
 // (unless its box is as large as the largest, in which case three) and 1.8
 // for an edge of two, whose cells hold eight times the space.  Two wins where
 // the lookups outnumber the records read, which the evaluation before tells
-// (it changes the time only, never the pairs).  The bounds lie a factor apart
-// so that the choice does not alternate.
+// (it changes the time only, never the pairs).  Records read a capsule with an
+// edge of two, and a step's time with an edge of one and of two, in us: 8.4:
+// 332 and 265, 11.4: 84 and 69, 18.8: 582 and 445, 42: 396 and 397, 54: 558 and
+// 572, 213: 1316 and 1500, 670: 2765 and 3157; so the line to an edge of one is
+// at 48.  An edge of one reads 2.4 times fewer; the line back, at 8 of them
+// (19 with an edge of two), lies well below so that the choice does not
+// alternate.
 __device__ __forceinline__ int32_t choose_edge(const ContactArgs& a) {
   const int32_t before = a.grid->edge_before;
   const unsigned long long n = static_cast<unsigned long long>(a.n_caps);
@@ -663,6 +668,9 @@ __device__ __forceinline__ void take_groups(uint32_t* taken, uint32_t n, Body&& 
 // a grid of resident CTAs whose warps take the entries (pass 0) or whose
 // threads step through the slots (pass 1, which leaves at once when no
 // capsule overflowed)
+// (At four CTAs an SM the search has 64 registers a thread and spills 172 B of
+// stores and 180 of loads, of both searches' bodies together; at three CTAs and
+// 80 registers it was 0 to 16 % slower.)
 template <int kPass>
 __global__ void __launch_bounds__(kThreads, 4) pairs_kernel(const ContactArgs a) {
   grid_dependency_wait();

@@ -571,7 +571,7 @@ eb_status setup_contact(eb_sim* s) {
   // (contact step 0.646 -> 0.633 ms against two a capsule; eight: 0.645 ms)
   while (table < 4 * n_caps) table <<= 1;
   c.table_mask = static_cast<uint32_t>(table - 1);
-  c.max_cells = static_cast<uint32_t>(2 * table);  // a dense grid of up to eight cells a capsule
+  c.max_cells = static_cast<uint32_t>(2 * table);  // a dense grid of 8 to 16 cells a capsule
   c.capacity = std::max<int64_t>(int64_t(1) << 16, 4 * n_caps);  // overflow lists only
   const size_t nm = s->materials.size();
   std::vector<eb::ContactPair> pairs(nm * nm);

@@ -635,7 +635,7 @@ cudaError_t launch_rod_block_mixed_pairs(const StepArgs& args, const int64_t* ct
 // Resident launches: CTA c owns the slots gmap[cta_start[c] .. cta_start[c +
 // 1]), whole rods (the host packs them best fit decreasing).  The same
 // configurations as the FP64 resident kernel (0/1: 520 slots, 2: 264, 3:
-// 320); 304 B of shared memory per slot (312 with explicit damping) allows
+// 320); 336 B of shared memory per slot (kMixedSlotBytes) allow
 // two CTAs per SM at 264 and 320 slots (two of 352 slots on 352 threads
 // measured 1% slower than 320 on the mixed batch).
 cudaError_t launch_rod_block_mixed_gather(const StepArgs& args, const int64_t* cta_start, const int32_t* gmap,

@@ -456,7 +456,12 @@ EB_API eb_status eb_partition_rods(const int64_t* weights, int64_t n, int32_t n_
  * by more than energy_tolerance times a scale (the sum of the initial energy
  * magnitudes plus m |g| L of every rod), or turns non-finite, are rerun in
  * FP64 from their initial conditions.  Rods of
- * a request hold at most 519 elements (one bin). */
+ * a request hold at most 1039 elements (a pair of bins).  Beside the pool the
+ * server keeps pinned host memory, 1 GiB for results on their way and 128 MiB
+ * for initial data; a request whose result is larger than the former (144
+ * bytes a node) cannot be delivered: it stays active, and every tick from the
+ * one that finishes it returns EB_ERR_OUT_OF_MEMORY after doing its work for
+ * the others. */
 typedef struct eb_server_config {
   int32_t device;
   int32_t precision;          /* EB_PRECISION_MIXED (with FP64 fallback) or EB_PRECISION_FP64 */
